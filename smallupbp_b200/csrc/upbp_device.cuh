@@ -57,6 +57,22 @@ __device__ __forceinline__ bool is_pos(float x) { return x > 1e-20f; }
 __device__ __forceinline__ bool rgb_positive(Rgb a) { return is_pos(a.r) && is_pos(a.g) && is_pos(a.b); }
 __device__ __forceinline__ bool rgb_black_or_neg(Rgb a) { return a.r <= 0.f && a.g <= 0.f && a.b <= 0.f; }
 
+// Reciprocal and reciprocal square root of the special function unit, one instruction each, for arguments
+// and results in the normal range.  Measured over [1, 4): root mean square error 3.0e-8 and 3.6e-8, mean
+// below 5e-9, as the approximate division (and a Newton step on the root makes its mean -1.5e-8).
+__device__ __forceinline__ float fast_rcp(float x)
+{
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+__device__ __forceinline__ float fast_rsqrt(float x)
+{
+    float r;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+
 // ------------------------------------------------------------------ media
 // HomogeneousMedium with its derived quantities (Scene/Media.hxx:129-159)
 struct DMedium {
@@ -283,6 +299,11 @@ __device__ __forceinline__ bool piece_takes_f64(V3 O1, V3 d1, float dmin, float 
     const double rho = (double)rs + sc.u * (double)rc + (double)extra;
     return sc.d2 <= rho * rho;
 }
+
+// Closest approach of a query's and a beam's line, as the mixed mode's contributions take it.
+struct PairGeo {
+    float cosb, distSqr, sinT, t1, u;  // d1.d2, squared distance, sin(theta), the lines' parameters
+};
 
 __device__ __forceinline__ bool piece_takes(V3 O1, V3 d1, float dmin, float dmax, V3 O2, V3 d2, float len,
                                             float t_lo, float t_hi, float t1, float b, float e, float dist, float rs,
