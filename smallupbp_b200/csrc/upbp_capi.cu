@@ -12,9 +12,9 @@
 
 #include "upbp_generic_api.cuh"
 #include "upbp_kdtree.cuh"
-#include "upbp_kdtree.cuh"
 #include "upbp_kernels.cuh"
 #include "upbp_mis_prep.cuh"
+#include "upbp_packet.cuh"
 #include "upbp_trace.cuh"
 
 using namespace upbp;
@@ -109,6 +109,8 @@ struct upbp_ctx {
     DBuf q_keys, q_keys_sorted, q_iota, q_order;
     // BB1D work order: the heavy queries (by PB2D candidate count) first
     DBuf bb_keys, bb_keys_sorted, bb_iota, bb_order, bb_sum;
+    // BB1D packets of camera rays (upbp_packet.cuh)
+    DBuf pk_range, pk_weight, pk_key, pk_key_sorted, pk_item, pk_item_sorted, pk_in, pk_totals;
     bool order_queries = true;
     int bm_n_leaves = 0;
     // mixed mode: FP64 partial sums of the MIS walks
@@ -136,6 +138,9 @@ struct upbp_ctx {
     int build_launches = 0, eval_launches = 0;
     float t_build = 0.f, t_pp3d = 0.f, t_pb2d = 0.f, t_bb1d = 0.f;
     cudaEvent_t ev[8] = {};
+    // the BB1D gather of the queries outside packets runs beside the packets' (created at first use)
+    cudaStream_t side_stream = nullptr;
+    cudaEvent_t fork = nullptr, join = nullptr;
 };
 
 namespace {
@@ -967,6 +972,43 @@ gen::GenLaunch generic_launch(upbp_ctx* c, const CamSum* cs_seg, const CamSum* c
     return A;
 }
 
+// The packets of camera rays in the pixel order, heaviest first (the heavy ones run for many times
+// the mean, and drawn last would run alone), and which queries they hold.
+PacketsDev find_packets(upbp_ctx* c, const SegQueriesDev& Q, const int32_t* order, const uint32_t* counts,
+                        float piece_len, int resident, cudaStream_t s)
+{
+    const int n = packet_blocks(c->P.image_width, c->P.image_height), slots = n * kPacketParts;
+    ensure(c, c->pk_range, sizeof(int2) * n);
+    ensure(c, c->pk_weight, sizeof(uint32_t) * n);
+    ensure(c, c->pk_key, sizeof(uint32_t) * slots);
+    ensure(c, c->pk_key_sorted, sizeof(uint32_t) * slots);
+    ensure(c, c->pk_item, sizeof(uint32_t) * slots);
+    ensure(c, c->pk_item_sorted, sizeof(uint32_t) * slots);
+    ensure(c, c->pk_in, (size_t)Q.n);
+    ensure(c, c->pk_totals, sizeof(PacketTotals));
+    ck(c, cudaMemsetAsync(c->pk_in.p, 0, (size_t)Q.n, s), "memset");
+    ck(c, cudaMemsetAsync(c->pk_totals.p, 0, sizeof(PacketTotals), s), "memset");
+    PacketsDev P{};
+    P.range = c->pk_range.as<int2>();
+    P.weight = c->pk_weight.as<uint32_t>();
+    P.key = c->pk_key.as<uint32_t>();
+    P.item = c->pk_item.as<uint32_t>();
+    P.item_sorted = c->pk_item_sorted.as<uint32_t>();
+    P.in_packet = c->pk_in.as<uint8_t>();
+    P.totals = c->pk_totals.as<PacketTotals>();
+    launch_packet_setup(Q, c->q_keys_sorted.as<uint32_t>(), order, counts, c->P.image_width, c->P.image_height,
+                        c->bbox_pc.as<float>(), piece_len, resident, P, s);
+    size_t b = 0;
+    cub::DeviceRadixSort::SortPairsDescending(nullptr, b, P.key, c->pk_key_sorted.as<uint32_t>(), P.item,
+                                              c->pk_item_sorted.as<uint32_t>(), slots, 0, 32, s);
+    ensure(c, c->cub_tmp, b);
+    ck(c, cub::DeviceRadixSort::SortPairsDescending(c->cub_tmp.p, b, P.key, c->pk_key_sorted.as<uint32_t>(), P.item,
+                                                    c->pk_item_sorted.as<uint32_t>(), slots, 0, 32, s),
+       "SortPairsDescending");
+    c->eval_launches += 6;
+    return P;
+}
+
 void record_status(upbp_ctx* c, cudaStream_t s)
 {
     if (!c->status_host) ck(c, cudaHostAlloc((void**)&c->status_host, sizeof(int), cudaHostAllocDefault),
@@ -1042,7 +1084,7 @@ void do_evaluate(upbp_ctx* c)
     const bool bp2d_warp = bp2d && c->pb2d_kernel == 1 && c->bb1d_kernel >= 1;
     if ((nq > 0 && (c->bb1d_kernel >= 1 || grid_mode)) || bp2d_warp) {
         // persistent warp kernels: work counters (BB1D or the fused kernel: [0], PB2D: [1],
-        // B-P2D: [2]) and the traversal status word they share
+        // B-P2D: [2], BB1D packets: [3]) and the traversal status word they share
         if (!c->num_sms) ck(c, cudaDeviceGetAttribute(&c->num_sms, cudaDevAttrMultiProcessorCount, c->device), "attr");
         ensure(c, c->work, sizeof(unsigned int) * 4);
         ensure(c, c->status, sizeof(int) * 4);
@@ -1090,7 +1132,21 @@ void do_evaluate(upbp_ctx* c)
     // count predicts it (both grow with the beam and photon density along the ray), so the
     // queries above kHeavyFactor x the mean PB2D count go first.
     const int32_t* bb_order = order;
-    if (order && nq > 1 && !fused && c->bb1d_kernel >= 1 && (c->P.techniques & UPBP_PB2D) && c->n_ph > 0) {
+    const bool counts = (c->P.techniques & UPBP_PB2D) && c->n_ph > 0;
+    // Camera rays in packets: they need the pixel order (its key holds 14 bits per axis), pieces, and
+    // enough packets to keep the blocks busy to the end: against one warp per query the packets take
+    // 0.6-0.8 of the time at 400 thousand queries and more, 0.7-1.0 at 100 thousand, and 1.0-1.3 below
+    // 70 thousand (cube, boxes and KNN scenes, measured either way).
+    constexpr int64_t kPacketQueries = 100000;
+    const bool packets = order && c->query_order == 1 && !fused && !grid_mode && c->bb1d_kernel >= 1 &&
+                         nq >= kPacketQueries && c->n_pieces > 0 && npix > 0 && c->P.image_width <= (1 << 14) &&
+                         c->P.image_height <= (1 << 14);
+    const float piece_len = std::max(1e-6f, c->piece_len_r * c->P.radius_bb1d);
+    const int packet_grid = packets ? c->num_sms * bb1d_packet_blocks_per_sm(mixed) : 0;
+    PacketsDev PK{};
+    if (packets)
+        PK = find_packets(c, Q, order, counts ? c->cnt_pb2d.as<uint32_t>() : nullptr, piece_len, packet_grid, s);
+    if (order && nq > 1 && !fused && c->bb1d_kernel >= 1 && (counts || packets)) {
         constexpr unsigned kHeavyFactor = 4;
         ensure(c, c->bb_keys, sizeof(uint32_t) * nq);
         ensure(c, c->bb_keys_sorted, sizeof(uint32_t) * nq);
@@ -1098,18 +1154,25 @@ void do_evaluate(upbp_ctx* c)
         ensure(c, c->bb_order, sizeof(int32_t) * nq);
         ensure(c, c->bb_sum, sizeof(unsigned long long));
         ck(c, cudaMemsetAsync(c->bb_sum.p, 0, sizeof(unsigned long long), s), "memset");
-        launch_heavy_keys(c->cnt_pb2d.as<uint32_t>(), nq, c->bb_sum.as<unsigned long long>(), kHeavyFactor,
-                          c->q_keys.as<uint32_t>(), c->bb_keys.as<uint32_t>(), c->bb_iota.as<int32_t>(), s);
+        launch_heavy_keys(counts ? c->cnt_pb2d.as<uint32_t>() : nullptr, nq, c->bb_sum.as<unsigned long long>(),
+                          kHeavyFactor, c->q_keys.as<uint32_t>(), PK.in_packet, c->bb_keys.as<uint32_t>(),
+                          c->bb_iota.as<int32_t>(), s);
         size_t b = 0;
         cub::DeviceRadixSort::SortPairs(nullptr, b, c->bb_keys.as<uint32_t>(), c->bb_keys_sorted.as<uint32_t>(),
-                                        c->bb_iota.as<int32_t>(), c->bb_order.as<int32_t>(), (int)nq, 0, 31, s);
+                                        c->bb_iota.as<int32_t>(), c->bb_order.as<int32_t>(), (int)nq, 0, 32, s);
         ensure(c, c->cub_tmp, b);
         ck(c, cub::DeviceRadixSort::SortPairs(c->cub_tmp.p, b, c->bb_keys.as<uint32_t>(),
                                               c->bb_keys_sorted.as<uint32_t>(), c->bb_iota.as<int32_t>(),
-                                              c->bb_order.as<int32_t>(), (int)nq, 0, 31, s),
+                                              c->bb_order.as<int32_t>(), (int)nq, 0, 32, s),
            "SortPairs");
         bb_order = c->bb_order.as<int32_t>();
         c->eval_launches += 4;
+    }
+    if (packets) {
+        if (!c->side_stream) ck(c, cudaStreamCreateWithFlags(&c->side_stream, cudaStreamNonBlocking), "stream");
+        if (!c->fork) ck(c, cudaEventCreateWithFlags(&c->fork, cudaEventDisableTiming), "event");
+        if (!c->join) ck(c, cudaEventCreateWithFlags(&c->join, cudaEventDisableTiming), "event");
+        ck(c, cudaEventRecord(c->fork, s), "fork");
     }
     if (nq > 0) {
         const BeamBVH B = beam_bvh(c);
@@ -1129,8 +1192,21 @@ void do_evaluate(upbp_ctx* c)
             record_status(c, s);
         } else if (c->bb1d_kernel >= 1) {
             const int grid = c->num_sms * bb1d_warp_blocks_per_sm(mixed, c->bb1d_kernel);
-            launch_bb1d_warp(K, L, B, S, Q, cam, cs_seg, O, grid, mixed, c->work.as<unsigned int>(),
-                             c->status.as<int>(), bb_order, s, c->bb1d_kernel);
+            if (packets) {
+                // The two gathers share no query.  The second stream lets the blocks of the per-query gather
+                // take the SMs that the last packets leave idle.
+                launch_bb1d_packet(K, L, B, S, Q, O, order, PK, c->bbox_pc.as<float>(), piece_len, packet_grid, mixed,
+                                   c->work.as<unsigned int>() + 3, s);
+                c->eval_launches += 1;
+                ck(c, cudaStreamWaitEvent(c->side_stream, c->fork, 0), "fork");
+                launch_bb1d_warp(K, L, B, S, Q, cam, cs_seg, O, grid, mixed, c->work.as<unsigned int>(),
+                                 c->status.as<int>(), bb_order, c->side_stream, c->bb1d_kernel, &PK.totals->queries);
+                ck(c, cudaEventRecord(c->join, c->side_stream), "join");
+                ck(c, cudaStreamWaitEvent(s, c->join, 0), "join");
+            } else {
+                launch_bb1d_warp(K, L, B, S, Q, cam, cs_seg, O, grid, mixed, c->work.as<unsigned int>(),
+                                 c->status.as<int>(), bb_order, s, c->bb1d_kernel, nullptr);
+            }
             record_status(c, s);
         } else {
             launch_gather_bb1d(K, L, B, S, Q, cam, cs_seg, O, c->block, mixed, s);
@@ -1219,11 +1295,15 @@ int upbp_ctx_destroy(upbp_ctx* c)
                    &c->gr_keys, &c->gr_keys_sorted, &c->gr_keys_unique, &c->gr_num, &c->gr_cellcount,
                    &c->gr_cells, &c->gr_ptr, &c->gr_pdf, &c->gr_draws, &c->gr_draw_off, &c->gr_rnd,
                    &c->gr_rec_a, &c->gr_rec_b, &c->gr_pay, &c->kd_qpts, &c->kd_qcodes, &c->kd_qcodes_sorted,
-                   &c->kd_qidx, &c->kd_qidx_sorted, &c->kd_qd2};
+                   &c->kd_qidx, &c->kd_qidx_sorted, &c->kd_qd2, &c->pk_range, &c->pk_weight,
+                   &c->pk_key, &c->pk_key_sorted, &c->pk_item, &c->pk_item_sorted, &c->pk_in, &c->pk_totals};
     for (DBuf* b : all) free_buf(*b);
     if (c->status_host) cudaFreeHost(c->status_host);
     for (auto& e : c->ev)
         if (e) cudaEventDestroy(e);
+    if (c->fork) cudaEventDestroy(c->fork);
+    if (c->join) cudaEventDestroy(c->join);
+    if (c->side_stream) cudaStreamDestroy(c->side_stream);
     if (c->own_stream) cudaStreamDestroy(c->own_stream);
     delete c;
     return UPBP_OK;

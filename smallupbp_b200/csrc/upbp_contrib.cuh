@@ -1,8 +1,8 @@
-// Contributions of the estimators, used by the gather kernels (upbp_gather.cu).
+// Contributions of the estimators, shared by the gather kernels (upbp_gather.cu, upbp_packet.cu).
 //
 //  * PB2D  : breIntersectFuncHomogeneous2 (Bre/Bre.cxx:293-464)
 //  * BB1D  : PhotonBeam::accumulate2 (Beams/PhotonBeam.hxx:386-607)
-// and the per-segment driver of evalBre / evalBeamBeamEstimate.  The file is compiled with the
+// and the per-segment driver of evalBre / evalBeamBeamEstimate.  Both files are compiled with the
 // approximate FP32 division; the candidate predicates use explicit IEEE intrinsics.
 #pragma once
 
@@ -209,6 +209,35 @@ __device__ __forceinline__ void closest_approach_f64(V3 O1, V3 d1, V3 O2, V3 d2,
     sinT = (float)s;
 }
 
+// Radius of a beam at t in the reference's operations (PhotonBeam.hxx:411); rc = 0: constant.
+__device__ __forceinline__ float radius_at(float rs, float rc, float t)
+{
+    return rc == 0.f ? rs : __fadd_rn(rs, __fmul_rn(t, rc));
+}
+
+// How far beyond its piece's interval the lines' closest point may lie, times sin(theta): 0 for an inner
+// piece; the first and the last piece also own the pairs whose closest point is clamped to the beam's end,
+// which the query's line then passes within the reach (the largest radius plus the margin).
+__device__ __forceinline__ float piece_slack(float len, float r2max, float t_lo, float t_hi, float extra)
+{
+    return t_lo > 0.f && t_hi < len ? 0.f : (r2max * fast_rsqrt(r2max) + extra) * 1.01f;
+}
+
+// The decision on a pair that bb1d_pair_fast leaves open (mixed mode): the reference's FP32 predicate
+// and radius test, the owner and the reach rule, in FP64 where FP32 does not decide, with the predicate's
+// closest approach or, for nearly parallel lines, the FP64 one.  Returns 1 or 0.
+__device__ __forceinline__ int pair_slow(V3 O1, V3 d1, float dmin, float dmax, V3 O2, V3 d2, float len, float r2max,
+                                         float t_lo, float t_hi, float rs, float rc, float extra, PairGeo& g)
+{
+    float dist, sinT, t1, t2, b, e;
+    if (!test_beam_beam(O1, d1, dmin, dmax, O2, d2, 0.f, len, r2max, &dist, &sinT, &t1, &t2, &b, &e)) return 0;
+    if (radius_at(rs, rc, t2) < dist) return 0;  // PhotonBeam.hxx:411-413
+    if (!piece_takes(O1, d1, dmin, dmax, O2, d2, len, t_lo, t_hi, t1, b, e, dist, rs, rc, extra)) return 0;
+    if (1.f - b * b < 1e-2f) closest_approach_f64(O1, d1, O2, d2, dist, sinT, t1, t2);
+    g = PairGeo{b, dist, sinT, t1, t2};
+    return 1;
+}
+
 template <bool kMixed>
 __device__ Rgb bb1d_contrib(const GatherConsts& K, const DMedium& m, const LightSoA& Lv, const BeamSoA& Bs,
                             const SegCtx& s, int beam, V3 bo, V3 bdir, float radius, float dist, float sinTheta,
@@ -306,13 +335,15 @@ __device__ Rgb bb1d_contrib(const GatherConsts& K, const DMedium& m, const Light
 }
 
 // PhotonBeam::accumulate2 (mixed mode) with the beam's payload packed per piece, at the lines' closest
-// approach g.  Reciprocals of the special function unit in place of the divisions, and fewer of them:
+// approach g.  kDirect: a camera path of length 1 (s.L is not read), which has no MIS records before the
+// merged vertex.  Reciprocals of the special function unit in place of the divisions, and fewer of them:
 // the kernel has one denominator, and the beam's side of the weight is arranged so that neither the squared
 // distance D nor the reverse pdf R along the beam is divided by:
 //   wLight = last * pdfAInv * (D bptb + phase * cont * cos * (d R + e)) / rspB.
 // (No constant is inverted beforehand: its rounding would be the same in every pair.)
 // BB1D against the version with a division per term: cube1024 274.9 -> 262.8 ms, boxes3 434.4 -> 417.8 ms,
 // cube512 21.7 -> 20.7 ms; per-query error against FP64 unchanged (p50 2.6e-7, p99 6.7e-6 at cube512).
+template <bool kDirect>
 __device__ __forceinline__ Rgb bb1d_contrib_packed(const GatherConsts& K, const DMedium& m, const SegCtx& s,
                                                    const PiecePayload& py, const PairGeo& g, float radius)
 {
@@ -330,12 +361,12 @@ __device__ __forceinline__ Rgb bb1d_contrib_packed(const GatherConsts& K, const 
     constexpr float inv4pi = (1.f / UPBP_PI_F) * 0.25f;
     const float phase =
         fabsf(m.g) < 1e-3f ? inv4pi : (hd > 0.f ? inv4pi * (1.f - g2) * (fast_rcp(hd) * fast_rsqrt(hd)) : 0.f);
-    // (1 - d^2 / r^2) * 3 / (4 r sin(theta)) over one denominator
-    const float r2 = radius * radius;
-    const float scale = phase * 0.75f * (r2 - g.distSqr) * fast_rcp(r2 * (radius * g.sinT));
+    // (1 - x^2) * 3 / (4 r sin(theta)) with x = d / r, as (1 - x)(1 + x): no cancellation where d approaches r
+    const float x = g.dist * fast_rcp(radius);
+    const float scale = phase * 0.75f * ((1.f - x) * (1.f + x)) * fast_rcp(radius * g.sinT);
     const Rgb unweighted = Rgb{py.thr.x * m.ss[0], py.thr.y * m.ss[1], py.thr.z * m.ss[2]} * att * scale;
     if (P.techniques & UPBP_NO_MIS) return unweighted;
-    const int L = s.L;
+    const int L = kDirect ? 1 : s.L;
     const uint32_t length = (uint32_t)((int)(lvbits & kPayPathMask) + 1 + L);
     if (length > P.max_path_length || length < P.min_path_length || (L == 1 && g.t1 < P.min_dist_to_med) ||
         !rgb_positive(att) || phase <= 0.f || rgb_black_or_neg(unweighted))

@@ -300,10 +300,52 @@ __device__ __forceinline__ bool piece_takes_f64(V3 O1, V3 d1, float dmin, float 
     return sc.d2 <= rho * rho;
 }
 
-// Closest approach of a query's and a beam's line, as the mixed mode's contributions take it.
+// The candidate decision and the closest approach of one pair, for the mixed mode's packets: 1 = this piece
+// takes the pair, 0 = it does not, -1 = undecided (the exact radius test and the reach rule decide; nearly
+// parallel pairs too, which also need the FP64 closest approach).  The predicate and its t1 and t2 are
+// test_beam_beam's operations; d1O1 = d1.O1 is the ray's, w = O2 - O1.  The distance and the sine come from
+// one approximate reciprocal square root instead of a root and a division, so the radius test is left
+// open within errb of the radius (the bound of piece_takes_fast, twice) and in the last 0.3 % of it, where
+// the kernel 1 - d^2 / r^2 would magnify their rounding; the owner is decided as there, and the reach rule
+// holds: the closest points lie inside both segments.  scale: the largest coordinate or
+// length in play; w1 bounds |w|_1; the directions are of unit length to 2e-6.
 struct PairGeo {
-    float cosb, distSqr, sinT, t1, u;  // d1.d2, squared distance, sin(theta), the lines' parameters
+    float cosb, dist, sinT, t1, u;  // d1.d2, distance, sin(theta), the lines' parameters
 };
+__device__ __forceinline__ int bb1d_pair_fast(V3 O1, V3 d1, float d1O1, float dmin, float dmax, V3 O2, V3 d2, float len,
+                                              float r2max, float t_lo, float t_hi, float w1, float scale, float rs,
+                                              float rc, PairGeo& g)
+{
+    const V3 c = xcross3(d1, d2);
+    const float s2 = xdot3(c, c);
+    const float ad = xdot3(xsub3(O2, O1), c);
+    if (xmul(ad, ad) >= xmul(r2max, s2)) return 0;
+    const float b = xdot3(d1, d2);
+    const float m1 = xsub(xmul(b, b), 1.0f);
+    if (m1 < 1e-5f && m1 > -1e-5f) return 0;
+    const float d1O2 = xdot3(d1, O2);
+    const float e = xsub(xdot3(d2, O1), xdot3(d2, O2));
+    const float t1 = xdiv(xsub(xsub(d1O1, d1O2), xmul(b, e)), m1);
+    if (t1 <= dmin || t1 >= dmax) return 0;
+    const float t2 = xdiv(xsub(xadd(t1, d1O1), d1O2), b);
+    if (t2 <= 0.f || t2 >= len || isnan(t2)) return 0;
+    const float rsn = fast_rsqrt(s2), dist = fabsf(ad) * rsn;
+    g.cosb = b;
+    g.dist = dist;
+    g.sinT = s2 * rsn;
+    g.t1 = t1;
+    g.u = t2;
+    const float m = 6e-6f * scale * (rsn * rsn);
+    const float u = e + b * t1;
+    const float errb = 1.6e-6f * w1 * rsn + 6e-6f * dist + 2e-8f;
+    const float room = rs + fminf(u * rc, t2 * rc) - dist;
+    const bool inside = fminf(fminf(t1 - dmin, dmax - t1), fminf(u, len - u)) > m;
+    if (inside && fminf(u - t_lo, t_hi - u) < -m) return 0;
+    if (inside && fminf(u - t_lo, t_hi - u) > m && room > fmaxf(errb + fabsf(rc) * m, 0.003f * dist) &&
+        s2 > 0.01f)
+        return 1;
+    return -1;
+}
 
 __device__ __forceinline__ bool piece_takes(V3 O1, V3 d1, float dmin, float dmax, V3 O2, V3 d2, float len,
                                             float t_lo, float t_hi, float t1, float b, float e, float dist, float rs,

@@ -166,8 +166,8 @@ __device__ __forceinline__ Rgb bb1d_query_warp(const GatherConsts& K, const DMed
             const int beam = __float_as_int(pc.z);
             if (kMixed) {
                 const PiecePayload py = B.pay[i];
-                const PairGeo pg{s.d.x * pb.x + s.d.y * pb.y + s.d.z * pb.z, g.x * g.x, g.y, g.z, g.w};
-                part = part + bb1d_contrib_packed(K, m, s, py, pg, beam_radius_at(Bs, beam, py.lv.z, g.w));
+                const PairGeo pg{s.d.x * pb.x + s.d.y * pb.y + s.d.z * pb.z, g.x, g.y, g.z, g.w};
+                part = part + bb1d_contrib_packed<false>(K, m, s, py, pg, beam_radius_at(Bs, beam, py.lv.z, g.w));
             } else {
                 part = part + bb1d_contrib<false>(K, m, Lv, Bs, s, beam, v3(pa.x, pa.y, pa.z), v3(pb.x, pb.y, pb.z),
                                                   beam_radius_at(Bs, beam, beam_start_radius(Bs, &Bs.radius[beam]), g.w), g.x, g.y,
@@ -328,14 +328,16 @@ __device__ __forceinline__ Rgb pb2d_query_warp(const GatherConsts& K, const DMed
 }
 
 // BB1D, warp per query, persistent: warps draw query indices (in Morton order of the query
-// midpoints) from an atomic counter.
+// midpoints) from an atomic counter.  elsewhere: how many queries at the end of the order the packet
+// gather evaluates (NULL: none).
 template <bool kMixed, int kWarps, int kMinBlocks>
 __global__ void __launch_bounds__(kWarps * 32, kMinBlocks) k_bb1d_warp(const __grid_constant__ GatherConsts K, const LightSoA Lv,
                                                           const BeamBVH B, const BeamSoA Bs, const SegQueriesDev Q,
                                                           const upbp_mis* __restrict__ cam,
                                                           const CamSum* __restrict__ cs, const Outputs O,
                                                           unsigned int* __restrict__ work, int* __restrict__ status,
-                                                          const int32_t* __restrict__ order)
+                                                          const int32_t* __restrict__ order,
+                                                          const unsigned* __restrict__ elsewhere)
 {
     __shared__ DMedium media[UPBP_MAX_MEDIA];
     __shared__ int s_stack[kWarps][kWarpStack];
@@ -346,11 +348,12 @@ __global__ void __launch_bounds__(kWarps * 32, kMinBlocks) k_bb1d_warp(const __g
     stage_media(K, media);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const WarpScratch ws{s_stack[warp], s_leaves[warp], &s_queue[warp], lane, (1u << lane) - 1u};
+    const int64_t n_items = Q.n - (elsewhere ? (int64_t)*elsewhere : 0);
     for (;;) {
         unsigned qq = 0;
         if (lane == 0) qq = atomicAdd(work, 1u);
         const int64_t item = (int64_t)__shfl_sync(kFull, qq, 0);
-        if (item >= Q.n) break;
+        if (item >= n_items) break;
         const int64_t q = order ? (int64_t)__ldg(&order[item]) : item;
         Rgb acc = rgb(0.f);
         unsigned long long cnt = 0, h = 0, tested = 0;
@@ -913,8 +916,8 @@ __device__ __forceinline__ Rgb bb1d_query_grid(const GatherConsts& K, const DMed
                 // (the candidate decision above stays FP32)
                 const float cb = s.d.x * d2.x + s.d.y * d2.y + s.d.z * d2.z;
                 if (1.f - cb * cb < 1e-2f) closest_approach_f64(s.o, s.d, o2, d2, dist, sinT, t1, t2);
-                c = bb1d_contrib_packed(K, m, s, G.pay[b], PairGeo{cb, dist * dist, sinT, t1, t2},
-                                        beam_radius_at(Bs, b, rs, t2));
+                c = bb1d_contrib_packed<false>(K, m, s, G.pay[b], PairGeo{cb, dist, sinT, t1, t2},
+                                               beam_radius_at(Bs, b, rs, t2));
             } else {
                 c = bb1d_contrib<false>(K, m, Lv, Bs, s, b, o2, d2, radius, dist, sinT, t1, t2);
             }
@@ -1195,15 +1198,15 @@ int bb1d_warp_blocks_per_sm(bool mixed, int variant)
 void launch_bb1d_warp(const GatherConsts& K, const LightSoA& L, const BeamBVH& B, const BeamSoA& S,
                       const SegQueriesDev& Q, const upbp_mis* cam, const CamSum* cs, const Outputs& O, int grid,
                       bool mixed, unsigned int* work, int* status, const int32_t* order, cudaStream_t stream,
-                      int variant)
+                      int variant, const unsigned* elsewhere)
 {
     if (Q.n <= 0) return;
     if (variant == 2) {
-        if (mixed) k_bb1d_warp<true, 4, 7><<<grid, 128, 0, stream>>>(K, L, B, S, Q, cam, cs, O, work, status, order);
-        else k_bb1d_warp<false, 4, 7><<<grid, 128, 0, stream>>>(K, L, B, S, Q, cam, cs, O, work, status, order);
+        if (mixed) k_bb1d_warp<true, 4, 7><<<grid, 128, 0, stream>>>(K, L, B, S, Q, cam, cs, O, work, status, order, elsewhere);
+        else k_bb1d_warp<false, 4, 7><<<grid, 128, 0, stream>>>(K, L, B, S, Q, cam, cs, O, work, status, order, elsewhere);
     } else {
-        if (mixed) k_bb1d_warp<true, 4, 6><<<grid, 128, 0, stream>>>(K, L, B, S, Q, cam, cs, O, work, status, order);
-        else k_bb1d_warp<false, 4, 6><<<grid, 128, 0, stream>>>(K, L, B, S, Q, cam, cs, O, work, status, order);
+        if (mixed) k_bb1d_warp<true, 4, 6><<<grid, 128, 0, stream>>>(K, L, B, S, Q, cam, cs, O, work, status, order, elsewhere);
+        else k_bb1d_warp<false, 4, 6><<<grid, 128, 0, stream>>>(K, L, B, S, Q, cam, cs, O, work, status, order, elsewhere);
     }
 }
 
@@ -1317,23 +1320,26 @@ __global__ void k_sum_counts(const uint32_t* __restrict__ cnt, int64_t n, unsign
 
 // BB1D work order: the queries whose PB2D candidate count exceeds `factor` times the mean come
 // first (they are the heaviest BB1D queries too), each group in Morton order of the midpoints.
+// Without counts (cnt NULL) none is heavy.  The queries that packets hold (in_packet, or NULL) go last.
 __global__ void k_heavy_keys(const uint32_t* __restrict__ cnt, int64_t n, const unsigned long long* __restrict__ sum,
-                             unsigned factor, const uint32_t* __restrict__ morton, uint32_t* keys, int32_t* iota)
+                             unsigned factor, const uint32_t* __restrict__ morton,
+                             const uint8_t* __restrict__ in_packet, uint32_t* keys, int32_t* iota)
 {
     const int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (q >= n) return;
-    const bool heavy = (unsigned long long)cnt[q] * (unsigned long long)n > (unsigned long long)factor * *sum;
-    keys[q] = (heavy ? 0u : (1u << 30)) | morton[q];
+    const bool heavy = cnt && (unsigned long long)cnt[q] * (unsigned long long)n > (unsigned long long)factor * *sum;
+    keys[q] = in_packet && in_packet[q] ? 0xffffffffu : (heavy ? 0u : (1u << 30)) | morton[q];
     iota[q] = (int32_t)q;
 }
 }  // namespace
 
 void launch_heavy_keys(const uint32_t* cnt, int64_t n, unsigned long long* sum, unsigned factor,
-                       const uint32_t* morton, uint32_t* keys, int32_t* iota, cudaStream_t stream)
+                       const uint32_t* morton, const uint8_t* in_packet, uint32_t* keys, int32_t* iota,
+                       cudaStream_t stream)
 {
     if (n <= 0) return;
-    k_sum_counts<<<148 * 4, 256, 0, stream>>>(cnt, n, sum);
-    k_heavy_keys<<<(int)((n + 255) / 256), 256, 0, stream>>>(cnt, n, sum, factor, morton, keys, iota);
+    if (cnt) k_sum_counts<<<148 * 4, 256, 0, stream>>>(cnt, n, sum);
+    k_heavy_keys<<<(int)((n + 255) / 256), 256, 0, stream>>>(cnt, n, sum, factor, morton, in_packet, keys, iota);
 }
 
 void launch_piece_payload(const float4* pc, int n, const float4* bm_thr, const float4* bm_pdf, const int2* bm_link,

@@ -241,10 +241,12 @@ void launch_piece_payload(const float4* pc, int n, const float4* bm_thr, const f
                           const struct LightSum* sums, PiecePayload* out, cudaStream_t stream);
 void launch_query_keys(const SegQueriesDev& Q, const float* bbox, int mode, int image_width, uint32_t* keys,
                        int32_t* iota, cudaStream_t stream);
-// keys that put the queries with more than `factor` x the mean PB2D candidate count first, each
-// group in the given Morton order; *sum must be zero on entry
+// keys that put the queries with more than `factor` x the mean PB2D candidate count first (none
+// without counts), each group in the given Morton order, and those that packets hold last; *sum
+// must be zero on entry
 void launch_heavy_keys(const uint32_t* cnt, int64_t n, unsigned long long* sum, unsigned factor,
-                       const uint32_t* morton, uint32_t* keys, int32_t* iota, cudaStream_t stream);
+                       const uint32_t* morton, const uint8_t* in_packet, uint32_t* keys, int32_t* iota,
+                       cudaStream_t stream);
 int bb1d_warp_blocks_per_sm(bool mixed, int variant);
 int pb2d_warp_blocks_per_sm(bool mixed);
 void launch_pb2d_warp(const GatherConsts& K, const LightSoA& L, const PhotonBVH& P, const SegQueriesDev& Q,
@@ -285,7 +287,7 @@ void launch_grid_reduce(const uint32_t* cells, uint32_t n_cells, uint32_t max_be
 void launch_bb1d_warp(const GatherConsts& K, const LightSoA& L, const BeamBVH& B, const BeamSoA& S,
                       const SegQueriesDev& Q, const upbp_mis* cam, const CamSum* cs, const Outputs& O, int grid,
                       bool mixed, unsigned int* work, int* status, const int32_t* order, cudaStream_t stream,
-                      int variant);
+                      int variant, const unsigned* elsewhere);
 void launch_gather_bp2d(const GatherConsts& K, const BeamBVH& B, const BeamSoA& S, const PointQueriesDev& Q,
                         const Outputs& O, int block, cudaStream_t stream);
 int bp2d_warp_blocks_per_sm();
