@@ -54,16 +54,31 @@ __global__ void k_bbox_partial(const float4* __restrict__ pts, const int32_t* __
         for (int c = 0; c < 6; ++c) partial[6 * blockIdx.x + c] = s[c][0];
 }
 
-__global__ void k_bbox_final(const float* partial, int blocks, float* out)
+// One block: lane-strided minima and maxima of the partial boxes, then over the block.  (A single thread
+// took 70 us for the 1024 boxes of a large input, 16 us for 160; minima have no order.)
+__global__ void __launch_bounds__(kThreads) k_bbox_final(const float* __restrict__ partial, int blocks, float* out)
 {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
+    __shared__ float s[6][kThreads / 32];
     float v[6] = {FLT_MAX, FLT_MAX, FLT_MAX, -FLT_MAX, -FLT_MAX, -FLT_MAX};
-    for (int b = 0; b < blocks; ++b)
+    for (int b = threadIdx.x; b < blocks; b += kThreads)
         for (int c = 0; c < 3; ++c) {
             v[c] = fminf(v[c], partial[6 * b + c]);
             v[3 + c] = fmaxf(v[3 + c], partial[6 * b + 3 + c]);
         }
-    for (int c = 0; c < 6; ++c) out[c] = v[c];
+    for (int c = 0; c < 3; ++c)
+        for (int o = 16; o > 0; o >>= 1) {
+            v[c] = fminf(v[c], __shfl_xor_sync(0xffffffffu, v[c], o));
+            v[3 + c] = fmaxf(v[3 + c], __shfl_xor_sync(0xffffffffu, v[3 + c], o));
+        }
+    if ((threadIdx.x & 31) == 0)
+        for (int c = 0; c < 6; ++c) s[c][threadIdx.x >> 5] = v[c];
+    __syncthreads();
+    if (threadIdx.x < 6) {
+        const int c = threadIdx.x;
+        float r = s[c][0];
+        for (int w = 1; w < kThreads / 32; ++w) r = c < 3 ? fminf(r, s[c][w]) : fmaxf(r, s[c][w]);
+        out[c] = r;
+    }
 }
 
 // ---------------------------------------------------------------- PP3D hash grid
@@ -421,7 +436,7 @@ void launch_bbox_partial(const float4* pts, const int32_t* idx, int n, float* pa
 }
 void launch_bbox_final(const float* partial, int blocks, float* out, cudaStream_t s)
 {
-    k_bbox_final<<<1, 32, 0, s>>>(partial, blocks, out);
+    k_bbox_final<<<1, kThreads, 0, s>>>(partial, blocks, out);
 }
 void launch_hash_keys(const float4* lv_pos, const int32_t* ph_lv, int n, const float* bbox, float inv_cell, int cells,
                       uint32_t* keys, cudaStream_t s)
