@@ -25,8 +25,6 @@
 #include <cfloat>
 #include <cstdint>
 
-#include <cub/block/block_scan.cuh>
-
 #include "upbp_kdtree.cuh"
 
 namespace upbp {
@@ -211,13 +209,17 @@ __global__ void k_kd_level_warp(float4* __restrict__ org, float4* __restrict__ t
 }
 
 // one level, the segments of more than kBigSeg points: one block each.  pa, pb: position scratch
-// (the segment's own range of it).
+// (the segment's own range of it).  A top level is a few blocks that sweep their segments alone, so the
+// sweep is what counts: a thread takes kSplitItems points of it at a time, the warps compact them with
+// ballots, and one barrier per kSplitItems x 1024 points adds the warps' counts up (block scans of one
+// point per thread took the eleven levels of 361 k points 12.1 ms).
 __global__ void __launch_bounds__(kSplitThreads) k_kd_level_big(float4* __restrict__ org, float4* __restrict__ tree,
                                                                 float* __restrict__ boxes, int* __restrict__ pa,
                                                                 int* __restrict__ pb, int n, int first)
 {
-    using Scan = cub::BlockScan<int, kSplitThreads>;
-    __shared__ typename Scan::TempStorage scan_tmp;
+    constexpr int kSplitItems = 8, kWarps = kSplitThreads / 32;
+    static_assert(kWarps == 32, "a warp adds up the warps' counts");
+    __shared__ int s_count[2][kWarps];
     __shared__ int s_left, s_right, s_m;
     const int idx = first + blockIdx.x;
     int start, end;
@@ -226,7 +228,8 @@ __global__ void __launch_bounds__(kSplitThreads) k_kd_level_big(float4* __restri
     for (int c = 0; c < 6; ++c) box[c] = boxes[6 * idx + c];
     const int axis = kd_axis(box);
     const int median = kd_median(start, end);
-    const int tid = threadIdx.x;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const unsigned lt = (1u << lane) - 1u;
     if (tid == 0) {
         s_left = start;
         s_right = end;
@@ -239,28 +242,54 @@ __global__ void __launch_bounds__(kSplitThreads) k_kd_level_big(float4* __restri
         // A: ascending positions in [left, right] with key >= v (right is the last);
         // B: ascending positions in (left, right) with key <= v (the sequential loop takes them
         // from the right)
-        int na = 0, nb = 0;
-        for (int base = left; base <= right; base += kSplitThreads) {
-            const int i = base + tid;
-            const float key = i <= right ? axis_of(org[i], axis) : 0.f;
-            const int fa = (i <= right && key >= v) ? 1 : 0;
-            const int fb = (i > left && i < right && key <= v) ? 1 : 0;
-            int ra, rb, ta, tb;
-            Scan(scan_tmp).ExclusiveSum(fa, ra, ta);
+        int na = 0, nb = 0, turn = 0;
+        for (int base = left; base <= right; base += kSplitItems * kSplitThreads, turn ^= 1) {
+            const int at = base + warp * kSplitItems * 32 + lane;
+            unsigned ba[kSplitItems], bb[kSplitItems];
+            int mine = 0;  // A's count, B's << 16
+#pragma unroll
+            for (int k = 0; k < kSplitItems; ++k) {
+                const int i = at + k * 32;
+                const float key = i <= right ? axis_of(org[i], axis) : 0.f;
+                ba[k] = __ballot_sync(kAllLanes, i <= right && key >= v);
+                bb[k] = __ballot_sync(kAllLanes, i > left && i < right && key <= v);
+                mine += __popc(ba[k]) | (__popc(bb[k]) << 16);
+            }
+            if (lane == 0) s_count[turn][warp] = mine;
             __syncthreads();
-            Scan(scan_tmp).ExclusiveSum(fb, rb, tb);
-            __syncthreads();
-            if (fa) pa[start + na + ra] = i;
-            if (fb) pb[start + nb + rb] = i;
-            na += ta;
-            nb += tb;
+            int upto = s_count[turn][lane];
+            for (int d = 1; d < 32; d <<= 1) {
+                const int u = __shfl_up_sync(kAllLanes, upto, d);
+                if (lane >= d) upto += u;
+            }
+            const int all = __shfl_sync(kAllLanes, upto, 31);
+            const int before = __shfl_sync(kAllLanes, upto, warp) - mine;
+            int oa = start + na + (before & 0xffff), ob = start + nb + (before >> 16);
+#pragma unroll
+            for (int k = 0; k < kSplitItems; ++k) {
+                if (ba[k] >> lane & 1u) pa[oa + __popc(ba[k] & lt)] = at + k * 32;
+                if (bb[k] >> lane & 1u) pb[ob + __popc(bb[k] & lt)] = at + k * 32;
+                oa += __popc(ba[k]);
+                ob += __popc(bb[k]);
+            }
+            na += all & 0xffff;
+            nb += all >> 16;
         }
-        if (tid == 0) s_m = na;
         __syncthreads();
-        // m = the first k with A[k] >= B'[k], B'[k] = the k-th from the right of B, then `left`
-        for (int k = tid; k < na; k += kSplitThreads) {
-            const int bk = k < nb ? pb[start + nb - 1 - k] : left;
-            if (pa[start + k] >= bk) atomicMin(&s_m, k);
+        // m = the first k with A[k] >= B'[k], B'[k] = the k-th from the right of B, then `left`: A ascends
+        // and B' descends, so the test turns true once, at the latest at A's last entry
+        if (warp == 0) {
+            int lo = 0, hi = na - 1;
+            while (lo < hi) {
+                const int step = (hi - lo + 32) / 32;  // 32 probes reach hi
+                const int k = min(lo + step * (lane + 1) - 1, hi);
+                const bool hit = pa[start + k] >= (k < nb ? pb[start + nb - 1 - k] : left);
+                const unsigned vote = __ballot_sync(kAllLanes, hit);  // hi's lane is among them
+                const int f = __ffs(vote) - 1;
+                hi = min(lo + step * (f + 1) - 1, hi);
+                lo = lo + step * f;
+            }
+            if (lane == 0) s_m = lo;
         }
         __syncthreads();
         const int m = s_m;
@@ -282,12 +311,23 @@ __global__ void __launch_bounds__(kSplitThreads) k_kd_level_big(float4* __restri
 }
 
 // KNNQuery (KdTmpl.hxx:692-760) with _checkAddNearest (:600-687) and the builds' initial radius
-// sqrt(FLT_MAX) (Bre.cxx:44, PhBeams.cxx:48); returns dist2[1]
+// sqrt(FLT_MAX) (Bre.cxx:44, PhBeams.cxx:48); returns dist2[1].
+//
+// The reference prunes a subtree by the distance to its last splitting plane alone.  Here it is also
+// pruned by the distance to its cell (the squared distances to the last plane crossed on each axis, added
+// in the order of a point's), with the same result: until k + 1 points are in, the bound heap[0] is
+// FLT_MAX and nothing is pruned; after that the heap holds the k smallest of what it held and of the
+// points met since, and the bound only shrinks.  Every point of a cell has a squared distance of at least
+// the cell's, rounding included (differences, squares and sums of non-negative terms round
+// monotonically), so a pruned point could not have entered the heap.  (A beam's end point just above
+// the light's plane, with a million origins on it, visited 724,000 nodes by the planes alone, in one walk of
+// dependent loads that lasted 120 ms at cube1024.)  KNN builds: cube1024 192 -> 44 ms, cube512 24.8 -> 14.7 ms.
 __device__ float kd_knn_d2(const float4* __restrict__ tree, int n, V3 q, int k)
 {
     float heap[kMaxKnn + 1];
-    int s_index[64];
-    float s_d2[64];
+    int s_index[64];            // the child on the query's side
+    float s_d2[64], s_old[64];  // squared distance to the plane; the axis' distance before crossing it
+    float ox = 0.f, oy = 0.f, oz = 0.f;  // the current cell's squared distance, by axis
     const int half = n / 2 - 1;
     const float r0 = __fsqrt_rn(FLT_MAX);
     heap[0] = __fmul_rn(r0, r0);
@@ -348,16 +388,32 @@ __device__ float kd_knn_d2(const float4* __restrict__ tree, int n, V3 q, int k)
             ++level;
         }
         add(index);
-        int camefrom;
-        do {
-            camefrom = index;
+        for (;;) {
+            const int camefrom = index;
             index /= 2;
             --level;
             if (index == 0) return heap[1];
-        } while (s_d2[level] >= heap[0] || camefrom != s_index[level]);
-        add(index);
-        index = s_index[level] ^ 1;
-        ++level;
+            const bool near = camefrom == s_index[level];
+            if (near && s_d2[level] >= heap[0]) continue;
+            const int plane = __float_as_int(__ldg(&tree[index].w));
+            if (!near) {  // back from the far side
+                if (plane == 0) ox = s_old[level];
+                else if (plane == 1) oy = s_old[level];
+                else oz = s_old[level];
+                continue;
+            }
+            add(index);
+            const float d2 = s_d2[level];
+            const float cell = __fadd_rn(__fadd_rn(plane == 0 ? d2 : ox, plane == 1 ? d2 : oy), plane == 2 ? d2 : oz);
+            if (cell >= heap[0]) continue;
+            s_old[level] = plane == 0 ? ox : (plane == 1 ? oy : oz);
+            if (plane == 0) ox = d2;
+            else if (plane == 1) oy = d2;
+            else oz = d2;
+            index = s_index[level] ^ 1;
+            ++level;
+            break;
+        }
     }
 }
 
