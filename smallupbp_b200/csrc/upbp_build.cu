@@ -346,10 +346,11 @@ __global__ void k_bbox_beams_partial(const float* __restrict__ origin, const flo
         for (int c = 0; c < 6; ++c) partial[6 * blockIdx.x + c] = s[c][0];
 }
 
-// Morton code of every piece's midpoint (one thread per piece); perm = the identity.
+// Morton code of every piece's midpoint (one thread per piece), and its beam, which the emission below
+// reads instead of searching again; perm = the identity.
 __global__ void k_piece_codes(const float* __restrict__ origin, const float* __restrict__ dir,
                               const float* __restrict__ length, int64_t nb, const int32_t* __restrict__ offsets,
-                              int np, const float* __restrict__ bbox, uint32_t* codes, int32_t* perm)
+                              int np, const float* __restrict__ bbox, uint32_t* codes, int32_t* perm, int32_t* beam)
 {
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= np) return;
@@ -360,23 +361,32 @@ __global__ void k_piece_codes(const float* __restrict__ origin, const float* __r
     codes[p] = morton3(origin[3 * b] + dir[3 * b] * tm, origin[3 * b + 1] + dir[3 * b + 1] * tm,
                        origin[3 * b + 2] + dir[3 * b + 2] * tm, bbox);
     perm[p] = p;
+    beam[p] = b;
 }
 
 // The records of the pieces in Morton order (one thread per sorted position): piece perm[i] of
 // its beam, at position i.  rstart / rchange / r2max (KNN radii, or NULL for the constant radius):
 // beam radius at t is rstart + t * rchange, the predicate's bound is r2max (PhotonBeam.hxx:238-296,
 // 411).
-__global__ void k_emit_sorted(const float* __restrict__ origin, const float* __restrict__ dir,
-                              const float* __restrict__ length, const int32_t* __restrict__ medium, int64_t nb,
-                              const int32_t* __restrict__ offsets, const int32_t* __restrict__ perm, int np,
-                              float radius, float eps, const float* __restrict__ rstart,
-                              const float* __restrict__ rchange, const float* __restrict__ r2max, float4* pa,
-                              float4* pb, float4* pc, Box* boxes)
+//
+// leaf <= 32: the boxes of the leaves (`leaf` consecutive positions, so neighbouring lanes) are reduced here
+// and only they are written, which saves the pieces' boxes a trip through memory; larger leaves: the
+// pieces' boxes.  payload (per beam) and pay (per piece): the beams' payloads copied into the order, or
+// NULL.  With a binary search for the beam, the pieces' boxes through memory and a gather of each piece's
+// payload from four arrays the build took 2.20 ms at cube512 (0.5 M pieces) and 14.8 ms at boxes3, now 1.59
+// and 9.7 ms.
+__global__ void __launch_bounds__(kThreads) k_emit_sorted(
+    const float* __restrict__ origin, const float* __restrict__ dir, const float* __restrict__ length,
+    const int32_t* __restrict__ medium, const int32_t* __restrict__ beam_of, const int32_t* __restrict__ offsets,
+    const int32_t* __restrict__ perm, int np, int leaf, float radius, float eps, const float* __restrict__ rstart,
+    const float* __restrict__ rchange, const float* __restrict__ r2max, const PiecePayload* __restrict__ payload,
+    float4* pa, float4* pb, float4* pc, PiecePayload* pay, Box* boxes)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= np) return;
-    const int p = perm[i];
-    const int b = piece_beam(offsets, nb, p);
+    const bool live = i < np;
+    if (leaf > 32 && !live) return;
+    const int p = perm[live ? i : np - 1];
+    const int b = beam_of[p];
     const int first = offsets[b], cnt = offsets[b + 1] - first, k = p - first;
     const float ox = origin[3 * b], oy = origin[3 * b + 1], oz = origin[3 * b + 2];
     const float dx = dir[3 * b], dy = dir[3 * b + 1], dz = dir[3 * b + 2];
@@ -412,10 +422,23 @@ __global__ void k_emit_sorted(const float* __restrict__ origin, const float* __r
         bx_.lo[1] = fminf(bx_.lo[1], by - re); bx_.hi[1] = fmaxf(bx_.hi[1], by + re);
         bx_.lo[2] = fminf(bx_.lo[2], bz - re); bx_.hi[2] = fmaxf(bx_.hi[2], bz + re);
     }
-    pa[i] = make_float4(ox, oy, oz, len);
-    pb[i] = make_float4(dx, dy, dz, r2);
-    pc[i] = make_float4(t0, t1, __int_as_float(b), __int_as_float(medium[b]));
-    boxes[i] = bx_;
+    if (live) {
+        pa[i] = make_float4(ox, oy, oz, len);
+        pb[i] = make_float4(dx, dy, dz, r2);
+        pc[i] = make_float4(t0, t1, __int_as_float(b), __int_as_float(medium[b]));
+        if (pay) pay[i] = payload[b];
+    }
+    if (leaf > 32) {
+        boxes[i] = bx_;
+        return;
+    }
+    // (the lanes past the end repeat the last piece, which changes no box)
+    for (int o = 1; o < leaf; o <<= 1)
+        for (int c = 0; c < 3; ++c) {
+            bx_.lo[c] = fminf(bx_.lo[c], __shfl_xor_sync(0xffffffffu, bx_.lo[c], o));
+            bx_.hi[c] = fmaxf(bx_.hi[c], __shfl_xor_sync(0xffffffffu, bx_.hi[c], o));
+        }
+    if (live && i % leaf == 0) boxes[i / leaf] = bx_;
 }
 
 }  // namespace
@@ -503,18 +526,21 @@ void launch_bbox_beams_partial(const float* origin, const float* dir, const floa
     k_bbox_beams_partial<<<blocks, kThreads, 0, s>>>(origin, dir, length, n, partial);
 }
 void launch_piece_codes(const float* origin, const float* dir, const float* length, int64_t nb, const int32_t* offsets,
-                        int np, const float* bbox, uint32_t* codes, int32_t* perm, cudaStream_t s)
-{
-    if (np > 0) k_piece_codes<<<blocks_for(np), kThreads, 0, s>>>(origin, dir, length, nb, offsets, np, bbox, codes, perm);
-}
-void launch_emit_sorted(const float* origin, const float* dir, const float* length, const int32_t* medium, int64_t nb,
-                        const int32_t* offsets, const int32_t* perm, int np, float radius, float eps,
-                        const float* rstart, const float* rchange, const float* r2max, float4* pa, float4* pb,
-                        float4* pc, Box* boxes, cudaStream_t s)
+                        int np, const float* bbox, uint32_t* codes, int32_t* perm, int32_t* beam, cudaStream_t s)
 {
     if (np > 0)
-        k_emit_sorted<<<blocks_for(np), kThreads, 0, s>>>(origin, dir, length, medium, nb, offsets, perm, np, radius,
-                                                          eps, rstart, rchange, r2max, pa, pb, pc, boxes);
+        k_piece_codes<<<blocks_for(np), kThreads, 0, s>>>(origin, dir, length, nb, offsets, np, bbox, codes, perm, beam);
+}
+void launch_emit_sorted(const float* origin, const float* dir, const float* length, const int32_t* medium,
+                        const int32_t* beam_of, const int32_t* offsets, const int32_t* perm, int np, int leaf, float radius,
+                        float eps, const float* rstart, const float* rchange, const float* r2max,
+                        const PiecePayload* payload, float4* pa, float4* pb, float4* pc, PiecePayload* pay, Box* boxes,
+                        cudaStream_t s)
+{
+    if (np > 0)
+        k_emit_sorted<<<blocks_for(np), kThreads, 0, s>>>(origin, dir, length, medium, beam_of, offsets, perm, np, leaf,
+                                                          radius, eps, rstart, rchange, r2max, payload, pa, pb, pc, pay,
+                                                          boxes);
 }
 
 }  // namespace upbp

@@ -87,11 +87,12 @@ struct upbp_ctx {
         pc_boxes2, pc_codes, pc_codes_sorted, pc_perm, pc_perm_sorted, bbox_pc;
     int n_pieces = 0;
     DBuf bm_leaf_codes, bm_nodes, bm_parent_int, bm_parent_leaf, bm_leaf_boxes, bm_node_boxes, bm_flagsbuf;
-    DBuf pc_pay;  // mixed mode: beam payload packed per piece
+    DBuf pc_pay, bm_pay;  // mixed mode: the contributions' inputs, per piece and per beam
+    DBuf pc_beam;         // the beam of each piece, in beam order
     // BB1D over the reference's uniform grid (upbp_set_bb1d_grid)
     upbp_bb1d_grid bgrid{};
     DBuf gr_hdr, gr_partial, gr_counts, gr_offsets, gr_keys, gr_keys_sorted, gr_keys_unique, gr_num, gr_cellcount,
-        gr_cells, gr_ptr, gr_pdf, gr_draws, gr_draw_off, gr_rnd, gr_rec_a, gr_rec_b, gr_pay;
+        gr_cells, gr_ptr, gr_pdf, gr_draws, gr_draw_off, gr_rnd, gr_rec_a, gr_rec_b;
     GridHeader gr_host{};           // the last build's header
     int64_t gr_raw = 0, gr_pairs = 0, gr_draws_total = 0;  // its sizes (a replay reuses them)
     bool gr_valid = false;
@@ -701,7 +702,7 @@ void do_build(upbp_ctx* c)
         ensure(c, c->pc_a2, sizeof(float4) * np);
         ensure(c, c->pc_b2, sizeof(float4) * np);
         ensure(c, c->pc_c2, sizeof(float4) * np);
-        ensure(c, c->pc_boxes2, sizeof(Box) * np);
+        ensure(c, c->pc_beam, sizeof(int32_t) * np);
         ensure(c, c->pc_codes, sizeof(uint32_t) * np);
         ensure(c, c->pc_codes_sorted, sizeof(uint32_t) * np);
         ensure(c, c->pc_perm, sizeof(int32_t) * np);
@@ -717,40 +718,36 @@ void do_build(upbp_ctx* c)
         launch_bbox_final(partial, bblocks, c->bbox_pc.as<float>(), s);
         launch_piece_codes(c->b_origin.as<float>(), c->b_dir.as<float>(), c->b_len.as<float>(), nb,
                            c->bm_offsets.as<int32_t>(), np, c->bbox_pc.as<float>(), c->pc_codes.as<uint32_t>(),
-                           c->pc_perm.as<int32_t>(), s);
+                           c->pc_perm.as<int32_t>(), c->pc_beam.as<int32_t>(), s);
         sort_pairs(c, c->pc_codes.as<uint32_t>(), c->pc_codes_sorted.as<uint32_t>(), c->pc_perm.as<int32_t>(),
                    c->pc_perm_sorted.as<int32_t>(), np, 30);
-        const float eps = bb1d_box_eps(r);
-        launch_emit_sorted(c->b_origin.as<float>(), c->b_dir.as<float>(), c->b_len.as<float>(),
-                           c->b_med_in.as<int32_t>(), nb, c->bm_offsets.as<int32_t>(), c->pc_perm_sorted.as<int32_t>(),
-                           np, r, eps, rchange ? c->bm_radius.as<float>() : nullptr, rchange, r2max,
-                           c->pc_a2.as<float4>(), c->pc_b2.as<float4>(), c->pc_c2.as<float4>(), c->pc_boxes2.as<Box>(),
-                           s);
         const int leaf = std::max(1, c->bb1d_leaf);
         const int nl = (np + leaf - 1) / leaf;
         ensure(c, c->bm_leaf_boxes, sizeof(Box) * nl);
-        launch_box_leaf_boxes(c->pc_boxes2.as<Box>(), np, leaf, c->bm_leaf_boxes.as<Box>(), s);
+        if (leaf > 32) ensure(c, c->pc_boxes2, sizeof(Box) * np);
+        PiecePayload* payload = nullptr;
+        if (c->mode != UPBP_MODE_PLAIN) {
+            // without MIS the payload holds the beam's throughput, flags and radius only
+            ensure(c, c->bm_pay, sizeof(PiecePayload) * nb);
+            ensure(c, c->pc_pay, sizeof(PiecePayload) * np);
+            payload = c->bm_pay.as<PiecePayload>();
+            launch_beam_payload((int)nb, c->bm_thr4.as<float4>(), c->bm_pdf4.as<float4>(), c->bm_link.as<int2>(),
+                                c->bm_radius.as<float>(), mis ? c->lv_info4.as<int4>() : nullptr,
+                                mis ? c->lv_mis.as<upbp_mis>() : nullptr, mis ? c->light_sums.as<LightSum>() : nullptr,
+                                payload, s);
+            c->build_launches += 1;
+        }
+        const float eps = bb1d_box_eps(r);
+        launch_emit_sorted(c->b_origin.as<float>(), c->b_dir.as<float>(), c->b_len.as<float>(),
+                           c->b_med_in.as<int32_t>(), c->pc_beam.as<int32_t>(), c->bm_offsets.as<int32_t>(),
+                           c->pc_perm_sorted.as<int32_t>(), np, leaf, r, eps, rchange ? c->bm_radius.as<float>() : nullptr,
+                           rchange, r2max, payload, c->pc_a2.as<float4>(), c->pc_b2.as<float4>(), c->pc_c2.as<float4>(),
+                           payload ? c->pc_pay.as<PiecePayload>() : nullptr,
+                           leaf > 32 ? c->pc_boxes2.as<Box>() : c->bm_leaf_boxes.as<Box>(), s);
+        if (leaf > 32) launch_box_leaf_boxes(c->pc_boxes2.as<Box>(), np, leaf, c->bm_leaf_boxes.as<Box>(), s);
         build_lbvh(c, c->pc_codes_sorted.as<uint32_t>(), np, leaf, c->bm_leaf_codes, c->bm_nodes, c->bm_parent_int,
                    c->bm_parent_leaf, c->bm_leaf_boxes, c->bm_node_boxes, c->bm_flagsbuf, c->bm_n_leaves);
-        c->build_launches += 8;
-        if (c->mode != UPBP_MODE_PLAIN) {
-            ensure(c, c->pc_pay, sizeof(PiecePayload) * np);
-            // without MIS the payload holds the beam's throughput, flags and radius only
-            launch_piece_payload(c->pc_c2.as<float4>(), np, c->bm_thr4.as<float4>(), c->bm_pdf4.as<float4>(),
-                                 c->bm_link.as<int2>(), c->bm_radius.as<float>(),
-                                 mis ? c->lv_info4.as<int4>() : nullptr, mis ? c->lv_mis.as<upbp_mis>() : nullptr,
-                                 mis ? c->light_sums.as<LightSum>() : nullptr, c->pc_pay.as<PiecePayload>(), s);
-            c->build_launches += 1;
-            if (c->bgrid.grid_res > 0) {
-                // the grid gather's payload: one per beam (the piece payload's layout)
-                ensure(c, c->gr_pay, sizeof(PiecePayload) * nb);
-                launch_piece_payload(nullptr, (int)nb, c->bm_thr4.as<float4>(), c->bm_pdf4.as<float4>(),
-                                     c->bm_link.as<int2>(), c->bm_radius.as<float>(),
-                                     mis ? c->lv_info4.as<int4>() : nullptr, mis ? c->lv_mis.as<upbp_mis>() : nullptr,
-                                     mis ? c->light_sums.as<LightSum>() : nullptr, c->gr_pay.as<PiecePayload>(), s);
-                c->build_launches += 1;
-            }
-        }
+        c->build_launches += leaf > 32 ? 8 : 7;
         if (c->bgrid.grid_res > 0) build_grid(c, s, r, rchange ? c->bm_radius.as<float>() : nullptr, rchange);
     }
     mark(c, 1, s);
@@ -881,7 +878,7 @@ BeamGrid grid_dev(upbp_ctx* c)
     G.rec_a = c->gr_rec_a.as<float4>();
     G.rec_b = c->gr_rec_b.as<float4>();
     G.medium = c->b_med_in.as<int32_t>();
-    G.pay = c->mode != UPBP_MODE_PLAIN ? c->gr_pay.as<PiecePayload>() : nullptr;
+    G.pay = c->mode != UPBP_MODE_PLAIN ? c->bm_pay.as<PiecePayload>() : nullptr;
     return G;
 }
 
@@ -1294,7 +1291,7 @@ int upbp_ctx_destroy(upbp_ctx* c)
                    &c->bb_order, &c->bb_sum, &c->gr_hdr, &c->gr_partial, &c->gr_counts, &c->gr_offsets,
                    &c->gr_keys, &c->gr_keys_sorted, &c->gr_keys_unique, &c->gr_num, &c->gr_cellcount,
                    &c->gr_cells, &c->gr_ptr, &c->gr_pdf, &c->gr_draws, &c->gr_draw_off, &c->gr_rnd,
-                   &c->gr_rec_a, &c->gr_rec_b, &c->gr_pay, &c->kd_qpts, &c->kd_qcodes, &c->kd_qcodes_sorted,
+                   &c->gr_rec_a, &c->gr_rec_b, &c->pc_beam, &c->bm_pay, &c->kd_qpts, &c->kd_qcodes, &c->kd_qcodes_sorted,
                    &c->kd_qidx, &c->kd_qidx_sorted, &c->kd_qd2, &c->pk_range, &c->pk_weight,
                    &c->pk_key, &c->pk_key_sorted, &c->pk_item, &c->pk_item_sorted, &c->pk_in, &c->pk_totals};
     for (DBuf* b : all) free_buf(*b);

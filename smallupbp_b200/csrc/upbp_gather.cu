@@ -1242,15 +1242,14 @@ void launch_bb1d_warp(const GatherConsts& K, const LightSoA& L, const BeamBVH& B
 }
 
 namespace {
-__global__ void k_piece_payload(const float4* __restrict__ pc, int n, const float4* __restrict__ bm_thr,
-                                const float4* __restrict__ bm_pdf, const int2* __restrict__ bm_link,
-                                const float* __restrict__ bm_radius, const int4* __restrict__ lv_info,
-                                const upbp_mis* __restrict__ lv_mis, const LightSum* __restrict__ sums,
-                                PiecePayload* __restrict__ out)
+// The contributions' inputs of every beam; the emission of the pieces copies them into its order.
+__global__ void k_beam_payload(int n, const float4* __restrict__ bm_thr, const float4* __restrict__ bm_pdf,
+                               const int2* __restrict__ bm_link, const float* __restrict__ bm_radius,
+                               const int4* __restrict__ lv_info, const upbp_mis* __restrict__ lv_mis,
+                               const LightSum* __restrict__ sums, PiecePayload* __restrict__ out)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const int beam = pc ? __float_as_int(pc[i].z) : i;  // pc == NULL: one payload per beam
+    const int beam = blockIdx.x * blockDim.x + threadIdx.x;
+    if (beam >= n) return;
     const int lv = bm_link[beam].x;
     // without MIS (lv_info == nullptr) the beams need not have light vertices
     upbp_mis m{};
@@ -1271,7 +1270,7 @@ __global__ void k_piece_payload(const float4* __restrict__ pc, int n, const floa
                           ((bflags & UPBP_SHORT_BEAM) ? (unsigned)kPayShortBeam : 0u) |
                           ((brsf & UPBP_ORIGIN_IN_MEDIUM) ? kPayOriginInMedium : 0u);
     p.lv = make_float4(onDelta ? 0.f : fabsf(m.cos_theta_out), ls.bptb, bm_radius[beam], __int_as_float((int)bits));
-    out[i] = p;
+    out[beam] = p;
 }
 
 // Morton code of the middle of a segment query's span (10 bits per axis in the given box).
@@ -1373,13 +1372,13 @@ void launch_heavy_keys(const uint32_t* cnt, int64_t n, unsigned long long* sum, 
     k_heavy_keys<<<(int)((n + 255) / 256), 256, 0, stream>>>(cnt, n, sum, factor, morton, in_packet, keys, iota);
 }
 
-void launch_piece_payload(const float4* pc, int n, const float4* bm_thr, const float4* bm_pdf, const int2* bm_link,
-                          const float* bm_radius, const int4* lv_info, const upbp_mis* lv_mis, const LightSum* sums,
-                          PiecePayload* out, cudaStream_t stream)
+void launch_beam_payload(int n, const float4* bm_thr, const float4* bm_pdf, const int2* bm_link, const float* bm_radius,
+                         const int4* lv_info, const upbp_mis* lv_mis, const LightSum* sums, PiecePayload* out,
+                         cudaStream_t stream)
 {
     if (n > 0)
-        k_piece_payload<<<(n + 255) / 256, 256, 0, stream>>>(pc, n, bm_thr, bm_pdf, bm_link, bm_radius, lv_info, lv_mis,
-                                                             sums, out);
+        k_beam_payload<<<(n + 255) / 256, 256, 0, stream>>>(n, bm_thr, bm_pdf, bm_link, bm_radius, lv_info, lv_mis, sums,
+                                                            out);
 }
 
 void launch_query_keys(const SegQueriesDev& Q, const float* bbox, int mode, int image_width, uint32_t* keys,

@@ -222,11 +222,12 @@ void launch_piece_counts(const float* length, int64_t n, float piece_len, int32_
 void launch_bbox_beams_partial(const float* origin, const float* dir, const float* length, int64_t n, float* partial,
                                int blocks, cudaStream_t s);
 void launch_piece_codes(const float* origin, const float* dir, const float* length, int64_t nb, const int32_t* offsets,
-                        int np, const float* bbox, uint32_t* codes, int32_t* perm, cudaStream_t s);
-void launch_emit_sorted(const float* origin, const float* dir, const float* length, const int32_t* medium, int64_t nb,
-                        const int32_t* offsets, const int32_t* perm, int np, float radius, float eps,
-                        const float* rstart, const float* rchange, const float* r2max, float4* pa, float4* pb,
-                        float4* pc, Box* boxes, cudaStream_t s);
+                        int np, const float* bbox, uint32_t* codes, int32_t* perm, int32_t* beam, cudaStream_t s);
+void launch_emit_sorted(const float* origin, const float* dir, const float* length, const int32_t* medium,
+                        const int32_t* beam_of, const int32_t* offsets, const int32_t* perm, int np, int leaf, float radius,
+                        float eps, const float* rstart, const float* rchange, const float* r2max,
+                        const PiecePayload* payload, float4* pa, float4* pb, float4* pc, PiecePayload* pay, Box* boxes,
+                        cudaStream_t s);
 void launch_box_leaf_boxes(const Box* boxes, int n, int leaf, Box* leaf_boxes, cudaStream_t stream);
 
 struct CamSum;
@@ -236,9 +237,9 @@ void launch_gather_pb2d(const GatherConsts& K, const LightSoA& L, const PhotonBV
 void launch_gather_bb1d(const GatherConsts& K, const LightSoA& L, const BeamBVH& B, const BeamSoA& S,
                         const SegQueriesDev& Q, const upbp_mis* cam, const CamSum* cs, const Outputs& O, int block,
                         bool mixed, cudaStream_t stream);
-void launch_piece_payload(const float4* pc, int n, const float4* bm_thr, const float4* bm_pdf, const int2* bm_link,
-                          const float* bm_radius, const int4* lv_info, const upbp_mis* lv_mis,
-                          const struct LightSum* sums, PiecePayload* out, cudaStream_t stream);
+void launch_beam_payload(int n, const float4* bm_thr, const float4* bm_pdf, const int2* bm_link, const float* bm_radius,
+                         const int4* lv_info, const upbp_mis* lv_mis, const struct LightSum* sums, PiecePayload* out,
+                         cudaStream_t stream);
 void launch_query_keys(const SegQueriesDev& Q, const float* bbox, int mode, int image_width, uint32_t* keys,
                        int32_t* iota, cudaStream_t stream);
 // keys that put the queries with more than `factor` x the mean PB2D candidate count first (none
