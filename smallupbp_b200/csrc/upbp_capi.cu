@@ -92,9 +92,10 @@ struct upbp_ctx {
     // BB1D over the reference's uniform grid (upbp_set_bb1d_grid)
     upbp_bb1d_grid bgrid{};
     DBuf gr_hdr, gr_partial, gr_counts, gr_offsets, gr_keys, gr_keys_sorted, gr_keys_unique, gr_num, gr_cellcount,
-        gr_cells, gr_ptr, gr_pdf, gr_draws, gr_draw_off, gr_rnd, gr_rec_a, gr_rec_b;
+        gr_cells, gr_ptr, gr_pdf, gr_draws, gr_draw_off, gr_rnd, gr_line, gr_r2, gr_beam_a, gr_beam_b, gr_beam_line;
     GridHeader gr_host{};           // the last build's header
     int64_t gr_raw = 0, gr_pairs = 0, gr_draws_total = 0;  // its sizes (a replay reuses them)
+    float gr_r2c = 0.f;             // its mMaxRadiusSqr (constant radius)
     bool gr_valid = false;
     // KNN radii: per-photon radius^2 (leaf order); per-beam radius change and max radius^2 (the
     // start radius goes to bm_radius); the LBVH over beam origins for the beam KNN search
@@ -392,12 +393,18 @@ void build_grid(upbp_ctx* c, cudaStream_t s, float radius, const float* rstart, 
         c->build_launches += 5;
     }
     // the entries' beam geometry in the final cell order (after the shuffles)
-    ensure(c, c->gr_rec_a, sizeof(float4) * std::max<int64_t>(np, 1));
-    ensure(c, c->gr_rec_b, sizeof(float4) * std::max<int64_t>(np, 1));
-    launch_grid_records(c->gr_ptr.as<int32_t>(), np, org, dir, len,
-                        (c->P.bb1d_knn > 0) ? c->bm_r2max.as<float>() : nullptr, radius * radius,
-                        c->gr_rec_a.as<float4>(), c->gr_rec_b.as<float4>(), s);
-    c->build_launches += 1;
+    const float* r2max = c->P.bb1d_knn > 0 ? c->bm_r2max.as<float>() : nullptr;
+    c->gr_r2c = radius * radius;
+    ensure(c, c->gr_line, sizeof(float4) * std::max<int64_t>(np, 1));
+    if (r2max) ensure(c, c->gr_r2, sizeof(float) * std::max<int64_t>(np, 1));
+    ensure(c, c->gr_beam_a, sizeof(float4) * nb);
+    ensure(c, c->gr_beam_b, sizeof(float4) * nb);
+    ensure(c, c->gr_beam_line, sizeof(float4) * nb);
+    launch_grid_beams(org, dir, len, r2max, c->gr_r2c, nb, hdr, c->gr_beam_a.as<float4>(), c->gr_beam_b.as<float4>(),
+                      c->gr_beam_line.as<float4>(), s);
+    launch_grid_records(c->gr_ptr.as<int32_t>(), np, c->gr_beam_line.as<float4>(), r2max, c->gr_line.as<float4>(),
+                        c->gr_r2.as<float>(), s);
+    c->build_launches += 2;
     c->gr_valid = true;
 }
 
@@ -875,8 +882,11 @@ BeamGrid grid_dev(upbp_ctx* c)
     G.cells = c->gr_cells.as<uint32_t>();
     G.pdf = c->bgrid.max_beams_in_cell > 0 ? c->gr_pdf.as<float>() : nullptr;
     G.ptr = c->gr_ptr.as<int32_t>();
-    G.rec_a = c->gr_rec_a.as<float4>();
-    G.rec_b = c->gr_rec_b.as<float4>();
+    G.line = c->gr_line.as<float4>();
+    G.line_r2 = c->P.bb1d_knn > 0 ? c->gr_r2.as<float>() : nullptr;
+    G.r2 = c->gr_r2c;
+    G.beam_a = c->gr_beam_a.as<float4>();
+    G.beam_b = c->gr_beam_b.as<float4>();
     G.medium = c->b_med_in.as<int32_t>();
     G.pay = c->mode != UPBP_MODE_PLAIN ? c->bm_pay.as<PiecePayload>() : nullptr;
     return G;
@@ -1291,7 +1301,7 @@ int upbp_ctx_destroy(upbp_ctx* c)
                    &c->bb_order, &c->bb_sum, &c->gr_hdr, &c->gr_partial, &c->gr_counts, &c->gr_offsets,
                    &c->gr_keys, &c->gr_keys_sorted, &c->gr_keys_unique, &c->gr_num, &c->gr_cellcount,
                    &c->gr_cells, &c->gr_ptr, &c->gr_pdf, &c->gr_draws, &c->gr_draw_off, &c->gr_rnd,
-                   &c->gr_rec_a, &c->gr_rec_b, &c->pc_beam, &c->bm_pay, &c->kd_qpts, &c->kd_qcodes, &c->kd_qcodes_sorted,
+                   &c->gr_line, &c->gr_r2, &c->gr_beam_a, &c->gr_beam_b, &c->gr_beam_line, &c->pc_beam, &c->bm_pay, &c->kd_qpts, &c->kd_qcodes, &c->kd_qcodes_sorted,
                    &c->kd_qidx, &c->kd_qidx_sorted, &c->kd_qd2, &c->pk_range, &c->pk_weight,
                    &c->pk_key, &c->pk_key_sorted, &c->pk_item, &c->pk_item_sorted, &c->pk_in, &c->pk_totals};
     for (DBuf* b : all) free_buf(*b);

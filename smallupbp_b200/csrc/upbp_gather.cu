@@ -878,16 +878,14 @@ __device__ __forceinline__ void grid_walk(const GridHeader& h, V3 o, V3 d, float
     }
 }
 
-// The cells of one warp's walk waiting for their beams to be tested, and the (cell, entry) items
-// past the first check of the predicate waiting for the rest of it.
-constexpr int kGridQueue = 32, kGridNear = 64;
+// The items of one warp's walk past the first checks of the predicate, waiting for the rest of it: the
+// entry in the cell lists, the cell's t range and its selection pdf.
+constexpr int kGridQueue = 64;
+constexpr uint32_t kNoEntry = 0xffffffffu;
 struct GridQueue {
     float tmin[kGridQueue], tmax[kGridQueue], pdf[kGridQueue];
-    uint32_t begin[kGridQueue], beams[kGridQueue];
-    unsigned long long key[kGridQueue];  // the cell's draws (reductions 1-3)
-    uint32_t first[kGridQueue + 1];      // the first item of every queued cell; first[n] = all items
-    float ntmin[kGridNear], ntmax[kGridNear], npdf[kGridNear];
-    uint32_t nat[kGridNear];             // the item's entry in the cell lists
+    uint32_t at[kGridQueue];
+    __align__(16) float ray[3][8];  // the query's line for each axis (grid_maybe)
 };
 
 // The per-query draws of the OFFSET, RESAMPLE_FIXED and SAMPLED reductions (Grid.hxx:466-548).  The
@@ -906,14 +904,47 @@ __device__ __forceinline__ float grid_draw(unsigned long long key, uint32_t j)
     return (float)(splitmix64(key + (unsigned long long)j * 0xD1B54A32D192ED03ull) >> 40) * 0x1p-24f;
 }
 
-// BB1D of one query by one warp over the beam grid.  The walk runs on every lane alike and queues
-// the visited cells that hold beams (max_beams_in_cell items of an over-full cell of a reduced
-// grid, Grid.hxx:453-548); once 32 or more (cell, beam) items wait, the lanes take them 32 at a
-// time through the first checks of PhotonBeam::testIntersectionBeamBeam (the distance of the two
-// lines, then the closest point's t1 within the cell's t range), from the entries' packed geometry.
-// The items that pass them go to a second queue, whose 32-wide batches run the rest: the medium,
-// the whole predicate, the radius, and PhotonBeam::accumulate / accumulate2 (PhotonBeam.hxx:315-367,
-// 375-480) divided by the cell's selection pdf.
+// Whether PhotonBeam::testIntersectionBeamBeam may accept a beam within the query's t range [tmin, tmax]
+// of a cell: its first two checks (the lines' distance, t1 within the range), on the beam's line with a
+// direction d2 = (1, m, n) of length up to sqrt(3), without the division and with fused multiply-adds.  The
+// checks are wider than the rounding of both sides; with M = mag, the sum of the coordinates' bounds, and unit
+// directions (within 1e-6):
+//   ad = x . (d1 x d2) / |d2| differs from the reference's by at most 2e-6 M, taken as a = 4e-6 M, the squared
+//   sine by 6e-4 of it where the predicate does not reject the pair as near-parallel; ad'^2 < r^2 sin'^2 gives
+//   ad^2 <= (1 + 1/16) ad'^2 + 17 a^2 < 1.07 r^2 sin^2 + c0;
+//   t1 = k / s2, k = (x.d1) |d2|^2 - b (x.d2), s2 = |d1 x d2|^2: k differs by at most 1.2e-5 M and s2 by 9e-6,
+//   so a t1 in the range keeps k within [tmin s2, tmax s2] widened by slack + 1.2e-5 tmax, slack = 2.5e-5 M.
+// NaN and infinite bounds pass.  The whole predicate in the reference's order decides in `finish`.
+// ray: the query's line for each axis, [axis] = {o_a, o_u, o_v, d_a, d_u, d_v}, o relative to the box's middle.
+__device__ __forceinline__ bool grid_maybe(const float (*ray)[8], float4 line, float r2, float tmin, float tmax,
+                                           float slack, float c0)
+{
+    const float* f = ray[min(__float_as_int(line.z) & 3, 2)];
+    const float4 f0 = *reinterpret_cast<const float4*>(f);
+    const float2 f1 = *reinterpret_cast<const float2*>(f + 4);
+    const float m = line.z, n = line.w, da = f0.w, du = f1.x, dv = f1.y;
+    const float xa = -f0.x, xu = line.x - f0.y, xv = line.y - f0.z;
+    const float ca = fmaf(du, n, -(dv * m)), cu = fmaf(-da, n, dv), cv = fmaf(da, m, -du);
+    const float ad = fmaf(xa, ca, fmaf(xu, cu, xv * cv)), s2 = fmaf(ca, ca, fmaf(cu, cu, cv * cv));
+    const float b = fmaf(du, m, fmaf(dv, n, da)), dd = fmaf(m, m, fmaf(n, n, 1.f));
+    const float xd1 = fmaf(xa, da, fmaf(xu, du, xv * dv)), xd2 = fmaf(xu, m, fmaf(xv, n, xa));
+    const float k = fmaf(-b, xd2, xd1 * dd), sl = fmaf(1.2e-5f, tmax, slack);
+    return !(ad * ad > fmaf(1.07f * r2, s2, c0)) && !(k < fmaf(tmin, s2, -sl)) && !(k > fmaf(tmax, s2, sl));
+}
+
+// BB1D of one query by one warp over the beam grid.  The walk runs on every lane alike.  The entries of a
+// visited cell (max_beams_in_cell items of an over-full cell of a reduced grid, Grid.hxx:453-548) go 32 at a
+// time, one per lane, through the first checks of PhotonBeam::testIntersectionBeamBeam (grid_maybe: the distance
+// of the two lines, then the closest point's t1 within the cell's t range), on their 16-byte lines.  Whole
+// batches of consecutive entries are checked at once, the next batch's lines loaded ahead; a cell's last items
+// and the items of reduced cells wait in the lanes' registers until the warp is full.  What passes goes to a
+// queue in shared memory, whose 32-wide batches run the rest: the medium, the whole predicate, the radius, and
+// PhotonBeam::accumulate / accumulate2 (PhotonBeam.hxx:315-367, 375-480) divided by the cell's selection pdf.
+//
+// Bound by instruction issue and the loads' latency: at cube512 over a 64^3 grid a query checks 15,000 entries
+// and takes 1,260.  With the cells queued in shared memory, two 16-byte loads per entry, the predicate's own
+// checks and batches that ended with the queue 35.7 ms, now 29.0 ms (128^3: 36.3 -> 32.4, cube128 over 64^3:
+// 1.00 -> 0.76).  Cells' last entries as partly filled batches: 31.8 ms.
 template <bool kMixed>
 __device__ __forceinline__ Rgb bb1d_query_grid(const GatherConsts& K, const DMedium* media, const LightSoA& Lv,
                                                const BeamGrid& G, const GridHeader& hdr, const BeamSoA& Bs,
@@ -926,15 +957,38 @@ __device__ __forceinline__ Rgb bb1d_query_grid(const GatherConsts& K, const DMed
     const Rgb res = segment_loop(K, media, Q, q, s, [&](const DMedium& m) {
         Rgb part = rgb(0.f);
         const int mid = (int)(&m - media);
-        int qc = 0, nq = 0;  // queued cells and items past the first check (warp-uniform)
+        int held = 0, nq = 0;  // the lanes that hold an item, and items past the first checks (warp-uniform)
+        // the lane's item: its entry, the cell's t range and selection pdf, the entry's geometry
+        uint32_t at = kNoEntry;
+        float imin = 0.f, imax = 0.f, ipdf = 1.f;
+        float4 line = make_float4(0.f, 0.f, 0.f, 0.f);
+        float r2 = G.r2;
+        // the bounds of grid_maybe
+        float mag = fabsf(s.o.x) + fabsf(s.o.y) + fabsf(s.o.z);
+        for (int k = 0; k < 3; ++k) mag += fmaxf(fabsf(hdr.lo[k]), fabsf(hdr.hi[k]));
+        if (!(fabsf(s.d.x * s.d.x + s.d.y * s.d.y + s.d.z * s.d.z - 1.f) <= 1e-6f)) mag = __int_as_float(0x7f800000);
+        const float slack = 2.5e-5f * mag, c0 = 2.72e-10f * mag * mag;
+        __syncwarp();
+        if (lane < 3) {
+            const float o[3] = {s.o.x - 0.5f * (hdr.lo[0] + hdr.hi[0]), s.o.y - 0.5f * (hdr.lo[1] + hdr.hi[1]),
+                                s.o.z - 0.5f * (hdr.lo[2] + hdr.hi[2])};
+            float* f = gq.ray[lane];
+            f[0] = pick3(lane, o[0], o[1], o[2]);
+            f[1] = pick3(lane, o[1], o[2], o[0]);
+            f[2] = pick3(lane, o[2], o[0], o[1]);
+            f[3] = pick3(lane, s.d.x, s.d.y, s.d.z);
+            f[4] = pick3(lane, s.d.y, s.d.z, s.d.x);
+            f[5] = pick3(lane, s.d.z, s.d.x, s.d.y);
+        }
+        __syncwarp();
         auto finish = [&](int k) {
-            const uint32_t at = gq.nat[k];
+            const uint32_t at = gq.at[k];
             const int b = __ldg(&G.ptr[at]);
             if (__ldg(&G.medium[b]) != mid) return;  // mMedium == medium
-            const float4 a = __ldg(&G.rec_a[at]), bd = __ldg(&G.rec_b[at]);
+            const float4 a = __ldg(&G.beam_a[b]), bd = __ldg(&G.beam_b[b]);
             const V3 o2 = v3(a.x, a.y, a.z), d2 = v3(bd.x, bd.y, bd.z);
             float dist, sinT, t1, t2;
-            if (!test_beam_beam(s.o, s.d, gq.ntmin[k], gq.ntmax[k], o2, d2, 0.f, a.w, bd.w, &dist, &sinT, &t1, &t2))
+            if (!test_beam_beam(s.o, s.d, gq.tmin[k], gq.tmax[k], o2, d2, 0.f, a.w, bd.w, &dist, &sinT, &t1, &t2))
                 return;
             const float rs = beam_start_radius(Bs, kMixed ? &G.pay[b].lv.z : &Bs.radius[b]);
             const float radius = beam_radius_at(Bs, b, rs, t2);
@@ -952,68 +1006,29 @@ __device__ __forceinline__ Rgb bb1d_query_grid(const GatherConsts& K, const DMed
             } else {
                 c = bb1d_contrib<false>(K, m, Lv, Bs, s, b, o2, d2, radius, dist, sinT, t1, t2);
             }
-            const float pdf = gq.npdf[k];
+            const float pdf = gq.pdf[k];
             if (pdf != 1.f) c = c * __fdiv_rn(1.f, pdf);
             part = part + c;
         };
-        // the queued cells' items; final: also the last items past the first check
-        auto flush = [&](bool final) {
-            const uint32_t total = qc > 0 ? gq.first[qc] : 0u;
-            for (uint32_t base = 0; base < total || (final && nq > 0); base += 32) {
-                const uint32_t it = base + (uint32_t)lane;
-                bool near = false;
-                int e = 0;
-                uint32_t at = 0;
-                if (it < total) {
-                    while (e + 1 < qc && gq.first[e + 1] <= it) ++e;
-                    const uint32_t j = it - gq.first[e], begin = gq.begin[e], beams = gq.beams[e];
-                    // the entry of item j: intersectPresampled / intersectOffsetted / intersectFixedSampled /
-                    // intersectSampled (Grid.hxx:453-548); unreduced cells and PRESAMPLE: the j-th of the list
-                    at = begin + j;
-                    bool take = true;
-                    if (gq.pdf[e] != 1.f && hdr.reduction != 0) {
-                        if (hdr.reduction == 1) {
-                            const uint32_t off = (uint32_t)__fmul_rn(grid_draw(gq.key[e], 0), (float)beams);
-                            const uint32_t k = min(hdr.max_beams, beams - min(off, beams));
-                            at = j < k ? begin + off + j : begin + (j - k);
-                        } else if (hdr.reduction == 2) {
-                            at = begin + min((uint32_t)__fmul_rn(grid_draw(gq.key[e], j), (float)beams), beams - 1);
-                        } else {
-                            take = grid_draw(gq.key[e], j) < gq.pdf[e];
-                        }
-                    }
-                    if (take) {
-                        ++tested32;
-                        const float4 a = __ldg(&G.rec_a[at]), bd = __ldg(&G.rec_b[at]);
-                        const V3 o2 = v3(a.x, a.y, a.z), d2 = v3(bd.x, bd.y, bd.z);
-                        if (beam_beam_near(s.o, s.d, o2, d2, bd.w)) {
-                            // a beam near the query's line is listed in every cell it crosses along the
-                            // walk; only the cell holding the lines' closest point accepts it
-                            float b12, b1o1, b1o2, be, t1;
-                            near = beam_beam_t1(s.o, s.d, o2, d2, b12, b1o1, b1o2, be, t1) &&
-                                   !(t1 <= gq.tmin[e] || t1 >= gq.tmax[e]);
-                        }
-                    }
-                }
-                const unsigned bal = __ballot_sync(kFull, near);
-                if (near) {
-                    const int slot = nq + __popc(bal & lt);
-                    gq.ntmin[slot] = gq.tmin[e];
-                    gq.ntmax[slot] = gq.tmax[e];
-                    gq.npdf[slot] = gq.pdf[e];
-                    gq.nat[slot] = at;
-                }
-                nq += __popc(bal);
-                __syncwarp();
-                if (nq >= 32 || (final && base + 32 >= total && nq > 0)) {
-                    const int n = min(nq, 32);
-                    nq -= n;
-                    if (lane < n) finish(nq + lane);
-                    __syncwarp();
-                }
+        // 32 items through the first checks, those that pass into the queue; `last`: and the queue's last ones
+        auto check = [&](bool valid, uint32_t entry, float4 ln, float rr, float tmin, float tmax, float pdf, bool last) {
+            const bool near = valid && grid_maybe(gq.ray, ln, rr, tmin, tmax, slack, c0);
+            const unsigned bal = __ballot_sync(kFull, near);
+            if (near) {
+                const int slot = nq + __popc(bal & lt);
+                gq.tmin[slot] = tmin;
+                gq.tmax[slot] = tmax;
+                gq.pdf[slot] = pdf;
+                gq.at[slot] = entry;
             }
-            qc = 0;
-            __syncwarp();
+            nq += __popc(bal);
+            while (nq >= 32 || (last && nq > 0)) {
+                const int n = min(nq, 32);
+                nq -= n;
+                __syncwarp();
+                if (lane < n) finish(nq + lane);
+                __syncwarp();
+            }
         };
         // the reductions' draws of this query and segment
         const unsigned long long qkey =
@@ -1025,22 +1040,57 @@ __device__ __forceinline__ Rgb bb1d_query_grid(const GatherConsts& K, const DMed
             const float pdf = G.pdf ? __ldg(&G.pdf[cell]) : 1.f;
             // a reduced cell tests max_beams beams, SAMPLED draws for each of them
             const uint32_t n = (pdf != 1.f && hdr.reduction != 3) ? hdr.max_beams : beams;
-            if (n == 0) return;
-            if (lane == 0) {
-                if (qc == 0) gq.first[0] = 0;
-                gq.tmin[qc] = cmin;
-                gq.tmax[qc] = cmax;
-                gq.pdf[qc] = pdf;
-                gq.begin[qc] = begin;
-                gq.beams[qc] = beams;
-                gq.key[qc] = splitmix64(qkey + (unsigned long long)cell * 0x9E3779B97F4A7C15ull);
-                gq.first[qc + 1] = gq.first[qc] + n;
+            // whole batches of an unreduced cell: 32 consecutive entries, the next ones loaded ahead
+            const uint32_t whole = pdf == 1.f || hdr.reduction == 0 ? n & ~31u : 0u;
+            float4 ahead = line;
+            if (whole) ahead = __ldg(&G.line[begin + (uint32_t)lane]);
+            for (uint32_t pos = 0; pos < n;) {
+                if (pos < whole) {
+                    const uint32_t entry = begin + pos + (uint32_t)lane;
+                    const float4 ln = ahead;
+                    pos += 32;
+                    ++tested32;
+                    if (pos < whole) ahead = __ldg(&G.line[entry + 32]);
+                    check(true, entry, ln, G.line_r2 ? __ldg(&G.line_r2[entry]) : G.r2, cmin, cmax, pdf, false);
+                    continue;
+                }
+                // the last items of a cell wait in the lanes until 32 are there
+                const uint32_t j = pos + (uint32_t)(lane - held);
+                if (lane >= held && j < n) {
+                    // the entry of item j: intersectPresampled / intersectOffsetted / intersectFixedSampled /
+                    // intersectSampled (Grid.hxx:453-548); unreduced cells and PRESAMPLE: the j-th of the list
+                    at = begin + j;
+                    if (pdf != 1.f && hdr.reduction != 0) {
+                        const unsigned long long key = splitmix64(qkey + (unsigned long long)cell * 0x9E3779B97F4A7C15ull);
+                        if (hdr.reduction == 1) {
+                            const uint32_t off = (uint32_t)__fmul_rn(grid_draw(key, 0), (float)beams);
+                            const uint32_t k = min(hdr.max_beams, beams - min(off, beams));
+                            at = j < k ? begin + off + j : begin + (j - k);
+                        } else if (hdr.reduction == 2) {
+                            at = begin + min((uint32_t)__fmul_rn(grid_draw(key, j), (float)beams), beams - 1);
+                        } else if (!(grid_draw(key, j) < pdf)) {
+                            at = kNoEntry;
+                        }
+                    }
+                    imin = cmin;
+                    imax = cmax;
+                    ipdf = pdf;
+                    if (at != kNoEntry) {
+                        ++tested32;
+                        line = __ldg(&G.line[at]);
+                        if (G.line_r2) r2 = __ldg(&G.line_r2[at]);
+                    }
+                }
+                const int took = (int)min(n - pos, (uint32_t)(32 - held));
+                pos += (uint32_t)took;
+                held += took;
+                if (held == 32) {
+                    held = 0;
+                    check(at != kNoEntry, at, line, r2, imin, imax, ipdf, false);
+                }
             }
-            __syncwarp();
-            ++qc;
-            if (qc == kGridQueue || gq.first[qc] >= 32) flush(false);
         });
-        if (qc > 0 || nq > 0) flush(true);
+        if (held > 0 || nq > 0) check(lane < held && at != kNoEntry, at, line, r2, imin, imax, ipdf, true);
         return part;
     });
     cnt += cnt32;
@@ -1048,11 +1098,11 @@ __device__ __forceinline__ Rgb bb1d_query_grid(const GatherConsts& K, const DMed
     return res;
 }
 
-// Persistent, one warp per query from the atomic work queue.  Compiled for 7 blocks of 4 warps per
-// SM (72 registers): the walk and the first checks stream the cell entries and wait on their loads,
-// so resident warps matter more than the spills of the rare contribution path.
+// Persistent, one warp per query from the atomic work queue.  5 blocks of 4 warps per SM: 6 and 7, with more
+// spills, take 29.1 and 29.6 ms instead of 29.0 at cube512 over a 64^3 grid, 0.78 and 0.81 instead of 0.76 at
+// cube128.
 template <bool kMixed>
-__global__ void __launch_bounds__(128, 7) k_bb1d_grid(const __grid_constant__ GatherConsts K, const LightSoA Lv,
+__global__ void __launch_bounds__(128, 5) k_bb1d_grid(const __grid_constant__ GatherConsts K, const LightSoA Lv,
                                                   const BeamGrid G, const BeamSoA Bs, const SegQueriesDev Q,
                                                   const upbp_mis* __restrict__ cam, const CamSum* __restrict__ cs,
                                                   const Outputs O, unsigned int* __restrict__ work,

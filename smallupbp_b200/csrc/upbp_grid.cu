@@ -254,18 +254,42 @@ __global__ void k_grid_lists(const unsigned long long* __restrict__ keys, int64_
     }
 }
 
-// The beam geometry of every cell entry, in the cells' (final, shuffled) order: (origin, length) and
-// (direction, maximal radius squared).  The gather reads 32 consecutive entries with two coalesced
-// 16-byte loads per lane instead of scattered loads through the beam id.
-__global__ void k_grid_records(const int32_t* __restrict__ ptr, int64_t n, const float* __restrict__ origin,
-                               const float* __restrict__ dir, const float* __restrict__ length,
-                               const float* __restrict__ r2max, float r2c, float4* __restrict__ rec_a,
-                               float4* __restrict__ rec_b)
+// The beams' geometry for the predicate, and the line of each beam for the gather's first checks, which
+// need its 4 degrees of freedom only: with a the axis of the direction's largest component and (u, v) the
+// next two in order, the slopes (du/da, dv/da) and the point (u, v) where the line meets the plane through the
+// middle of the grid's box, relative to that middle.  a is in the last two bits of the first slope.  The
+// checks' bounds hold for a unit direction: another one (or a NaN) gets a NaN line, which passes every check.
+__global__ void k_grid_beams(const float* __restrict__ origin, const float* __restrict__ dir,
+                             const float* __restrict__ length, const float* __restrict__ r2max, float r2c, int64_t nb,
+                             const GridHeader* __restrict__ hdr, float4* __restrict__ beam_a,
+                             float4* __restrict__ beam_b, float4* __restrict__ line)
+{
+    const int64_t b = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (b >= nb) return;
+    const float o[3] = {origin[3 * b], origin[3 * b + 1], origin[3 * b + 2]};
+    const float d[3] = {dir[3 * b], dir[3 * b + 1], dir[3 * b + 2]};
+    beam_a[b] = make_float4(o[0], o[1], o[2], length[b]);
+    beam_b[b] = make_float4(d[0], d[1], d[2], r2max ? r2max[b] : r2c);
+    const int a = fabsf(d[0]) >= fabsf(d[1]) ? (fabsf(d[0]) >= fabsf(d[2]) ? 0 : 2) : (fabsf(d[1]) >= fabsf(d[2]) ? 1 : 2);
+    float c[3];
+    for (int k = 0; k < 3; ++k) c[k] = o[k] - 0.5f * (hdr->lo[k] + hdr->hi[k]);
+    const float oa = a == 0 ? c[0] : (a == 1 ? c[1] : c[2]), da = a == 0 ? d[0] : (a == 1 ? d[1] : d[2]);
+    const float ou = a == 0 ? c[1] : (a == 1 ? c[2] : c[0]), du = a == 0 ? d[1] : (a == 1 ? d[2] : d[0]);
+    const float ov = a == 0 ? c[2] : (a == 1 ? c[0] : c[1]), dv = a == 0 ? d[2] : (a == 1 ? d[0] : d[1]);
+    const float m = __int_as_float((__float_as_int(du / da) & ~3) | a), n = dv / da;
+    const float dd = d[0] * d[0] + d[1] * d[1] + d[2] * d[2];
+    const float p = fabsf(dd - 1.f) <= 1e-6f ? fmaf(-oa, m, ou) : __int_as_float(0x7fffffff);
+    line[b] = make_float4(p, fmaf(-oa, n, ov), m, n);
+}
+
+// the lines of the cell entries, in the final cell order
+__global__ void k_grid_records(const int32_t* __restrict__ ptr, int64_t n, const float4* __restrict__ line,
+                               const float* __restrict__ r2max, float4* __restrict__ rec, float* __restrict__ rec_r2)
 {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         const int b = ptr[i];
-        rec_a[i] = make_float4(origin[3 * b], origin[3 * b + 1], origin[3 * b + 2], length[b]);
-        rec_b[i] = make_float4(dir[3 * b], dir[3 * b + 1], dir[3 * b + 2], r2max ? r2max[b] : r2c);
+        rec[i] = line[b];
+        if (r2max) rec_r2[i] = r2max[b];
     }
 }
 
@@ -401,10 +425,16 @@ void launch_grid_lists(const unsigned long long* keys, int64_t n, uint32_t* coun
 {
     if (n > 0) k_grid_lists<<<blocks_for(n), kThreads, 0, s>>>(keys, n, counts, ptr);
 }
-void launch_grid_records(const int32_t* ptr, int64_t n, const float* origin, const float* dir, const float* length,
-                         const float* r2max, float r2c, float4* rec_a, float4* rec_b, cudaStream_t s)
+void launch_grid_beams(const float* origin, const float* dir, const float* length, const float* r2max, float r2c,
+                       int64_t nb, const GridHeader* hdr, float4* beam_a, float4* beam_b, float4* line, cudaStream_t s)
 {
-    if (n > 0) k_grid_records<<<blocks_for(n), kThreads, 0, s>>>(ptr, n, origin, dir, length, r2max, r2c, rec_a, rec_b);
+    if (nb > 0)
+        k_grid_beams<<<blocks_for(nb), kThreads, 0, s>>>(origin, dir, length, r2max, r2c, nb, hdr, beam_a, beam_b, line);
+}
+void launch_grid_records(const int32_t* ptr, int64_t n, const float4* line, const float* r2max, float4* rec,
+                         float* rec_r2, cudaStream_t s)
+{
+    if (n > 0) k_grid_records<<<blocks_for(n), kThreads, 0, s>>>(ptr, n, line, r2max, rec, rec_r2);
 }
 void launch_grid_draws(const uint32_t* cells, uint32_t n_cells, uint32_t max_beams, uint32_t reduction,
                        uint32_t* draws, cudaStream_t s)

@@ -88,8 +88,11 @@ struct BeamGrid {
     const uint32_t* cells;  // mCells: the first entry of every cell's list (n_cells entries)
     const float* pdf;       // mPdfs, NULL: 1 in every cell (no reduction)
     const int32_t* ptr;     // mPointers: beam ids, each cell's beams in descending id order
-    const float4* rec_a;    // per entry of ptr: the beam's origin xyz, length
-    const float4* rec_b;    // per entry of ptr: the beam's direction xyz, mMaxRadiusSqr
+    const float4* line;     // per entry of ptr: the beam's line (k_grid_beams)
+    const float* line_r2;   // per entry of ptr: mMaxRadiusSqr, NULL: r2 for all
+    float r2;
+    const float4* beam_a;   // per beam: origin xyz, length
+    const float4* beam_b;   // per beam: direction xyz, mMaxRadiusSqr
     const int32_t* medium;  // per beam, as uploaded
     const PiecePayload* pay;  // mixed mode: the contribution's inputs per beam (PiecePayload layout)
 };
@@ -277,8 +280,10 @@ void launch_grid_emit(const float* origin, const float* dir, const float* length
                       const float* rchange, float radius, int64_t nb, const GridHeader* hdr,
                       const unsigned long long* offsets, unsigned long long* keys, cudaStream_t s);
 void launch_grid_lists(const unsigned long long* keys, int64_t n, uint32_t* counts, int32_t* ptr, cudaStream_t s);
-void launch_grid_records(const int32_t* ptr, int64_t n, const float* origin, const float* dir, const float* length,
-                         const float* r2max, float r2c, float4* rec_a, float4* rec_b, cudaStream_t s);
+void launch_grid_beams(const float* origin, const float* dir, const float* length, const float* r2max, float r2c,
+                       int64_t nb, const GridHeader* hdr, float4* beam_a, float4* beam_b, float4* line, cudaStream_t s);
+void launch_grid_records(const int32_t* ptr, int64_t n, const float4* line, const float* r2max, float4* rec,
+                         float* rec_r2, cudaStream_t s);
 void launch_grid_draws(const uint32_t* cells, uint32_t n_cells, uint32_t max_beams, uint32_t reduction,
                        uint32_t* draws, cudaStream_t s);
 void launch_mt64_floats(unsigned long long seed, int64_t n, float* out, cudaStream_t s);
