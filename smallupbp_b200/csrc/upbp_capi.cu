@@ -330,10 +330,10 @@ void build_grid(upbp_ctx* c, cudaStream_t s, float radius, const float* rstart, 
     const int end_bit = 32 + bits_for(nc);
     b = 0;
     cub::DeviceRadixSort::SortKeys(nullptr, b, c->gr_keys.as<unsigned long long>(),
-                                   c->gr_keys_sorted.as<unsigned long long>(), (int)raw, 0, end_bit, s);
+                                   c->gr_keys_sorted.as<unsigned long long>(), (int)raw, 32, end_bit, s);
     ensure(c, c->cub_tmp, b);
     ck(c, cub::DeviceRadixSort::SortKeys(c->cub_tmp.p, b, c->gr_keys.as<unsigned long long>(),
-                                         c->gr_keys_sorted.as<unsigned long long>(), (int)raw, 0, end_bit, s),
+                                         c->gr_keys_sorted.as<unsigned long long>(), (int)raw, 32, end_bit, s),
        "SortKeys");
     b = 0;
     cub::DeviceSelect::Unique(nullptr, b, c->gr_keys_sorted.as<unsigned long long>(),
