@@ -336,13 +336,14 @@ __device__ Rgb bb1d_contrib(const GatherConsts& K, const DMedium& m, const Light
 
 // PhotonBeam::accumulate2 (mixed mode) with the beam's payload packed per piece, at the lines' closest
 // approach g.  kDirect: a camera path of length 1 (s.L is not read), which has no MIS records before the
-// merged vertex.  Reciprocals of the special function unit in place of the divisions, and fewer of them:
-// the kernel has one denominator, and the beam's side of the weight is arranged so that neither the squared
-// distance D nor the reverse pdf R along the beam is divided by:
+// merged vertex.  Fewer divisions, the others as reciprocals of the special function unit: one factor for the
+// three channels, and the beam's side of the weight arranged so that neither the squared distance D nor the
+// reverse pdf R along the beam is divided by:
 //   wLight = last * pdfAInv * (D bptb + phase * cont * cos * (d R + e)) / rspB.
 // (No constant is inverted beforehand: its rounding would be the same in every pair.)
-// BB1D against the version with a division per term: cube1024 274.9 -> 262.8 ms, boxes3 434.4 -> 417.8 ms,
-// cube512 21.7 -> 20.7 ms; per-query error against FP64 unchanged (p50 2.6e-7, p99 6.7e-6 at cube512).
+// BB1D against the version with a division per term, without packets: nested boxes with 300 x 300 pixels 4.74 ->
+// 4.49 ms, LONG beams with 256 x 200 pixels 2.98 -> 2.82 ms; per-query error against FP64 at cube512 p50
+// 2.56e-7 -> 2.58e-7, root mean square 1.325e-6 in both.
 template <bool kDirect>
 __device__ __forceinline__ Rgb bb1d_contrib_packed(const GatherConsts& K, const DMedium& m, const SegCtx& s,
                                                    const PiecePayload& py, const PairGeo& g, float radius)
@@ -360,10 +361,12 @@ __device__ __forceinline__ Rgb bb1d_contrib_packed(const GatherConsts& K, const 
     const float g2 = m.g * m.g, hd = 1.f + g2 + (m.g + m.g) * g.cosb;
     constexpr float inv4pi = (1.f / UPBP_PI_F) * 0.25f;
     const float phase =
-        fabsf(m.g) < 1e-3f ? inv4pi : (hd > 0.f ? inv4pi * (1.f - g2) * (fast_rcp(hd) * fast_rsqrt(hd)) : 0.f);
-    // (1 - x^2) * 3 / (4 r sin(theta)) with x = d / r, as (1 - x)(1 + x): no cancellation where d approaches r
-    const float x = g.dist * fast_rcp(radius);
-    const float scale = phase * 0.75f * ((1.f - x) * (1.f + x)) * fast_rcp(radius * g.sinT);
+        fabsf(m.g) < 1e-3f ? inv4pi : (hd > 0.f ? inv4pi * (1.f - g2) / (hd * sqrtf(hd)) : 0.f);
+    // one factor for the three channels.  The root and the kernel are as in the general form: with the two
+    // functions' product rcp(hd) rsqrt(hd) and (1 - x)(1 + x) * 0.75 / (r sin), 1.8 % faster, each rounding of a
+    // constant goes the same way for every pair, and the error against FP64 grew by up to 6.6 % (SHORT query
+    // beams), 3.1 % (nested boxes) and 1.2 % (cube128); now it is within 0.4 % to either side, 1.7 % for the first
+    const float scale = phase * (1.f - g.dist * g.dist / (radius * radius)) * 3.f / (4.f * radius * g.sinT);
     const Rgb unweighted = Rgb{py.thr.x * m.ss[0], py.thr.y * m.ss[1], py.thr.z * m.ss[2]} * att * scale;
     if (P.techniques & UPBP_NO_MIS) return unweighted;
     const int L = kDirect ? 1 : s.L;
