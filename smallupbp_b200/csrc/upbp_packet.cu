@@ -762,7 +762,9 @@ k_bb1d_packet(const __grid_constant__ GatherConsts K, const __grid_constant__ Li
                 }
                 __syncthreads();
             } while (!last);
-            if (warp == 0) {
+            // (a ray whose segments have ended may hold an attenuation that is no number, which segment_loop
+            // never uses)
+            if (warp == 0 && (S.walk.active >> lane & 1u)) {
                 S.sum_r[lane] += S.attn_r[lane] * S.acc_r[lane];
                 S.sum_g[lane] += S.attn_g[lane] * S.acc_g[lane];
                 S.sum_b[lane] += S.attn_b[lane] * S.acc_b[lane];

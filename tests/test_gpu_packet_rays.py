@@ -1,0 +1,95 @@
+"""BB1D over packets of camera rays (upbp_packet.cu), for ray records that a caller supplies: rays whose
+transmittance beyond their last segment is no number, wide fans of short rays, and coordinates far
+from the origin.  As in test_gpu_packets.py the order along the midpoints (query_order 0), which forms no
+packets, is the general path: both take the same pairs, so counts and hashes are equal."""
+import numpy as np
+import pytest
+
+import golden_io as G
+from smallupbp_b200 import engine
+from smallupbp_b200 import workload as W
+
+_made = {}
+
+
+def workload(**kw):
+    key = tuple(sorted(kw.items()))
+    if key not in _made:
+        _made[key] = W.generate(W.cube_scene("rays", 419, 317, 3000, 6, 0.01, **kw), 0)
+        assert len(_made[key]["sq_flags"]) >= 100000
+    return {k: v.copy() for k, v in _made[key].items()}
+
+
+def results(w, mode, **tuning):
+    with engine.EstimatorStage(0, mode) as st:
+        st.set_tuning(**tuning)
+        st.run(w)
+        return st.segment_results()[1], st.query_stats(), st.tested_counts()["bb1d"]
+
+
+def both(w, mode, **tuning):
+    got, s, tested = results(w, mode, query_order=1, **tuning)
+    want, s0, tested0 = results(w, mode, query_order=0, **tuning)
+    assert tested != tested0  # the packets ran
+    return got, s, want, s0
+
+
+def same_pairs(s, s0):
+    for k in ("count_bb1d", "hash_bb1d"):
+        np.testing.assert_array_equal(s[k], s0[k], err_msg=k)
+
+
+def set_segments(w, q, segments, flags=None):
+    """The segments (dmin, dmax, medium, pdf, attenuation) of query q, appended to the arrays' lists."""
+    w["sq_seg_begin"][q] = len(w["seg_dist_min"])
+    w["sq_seg_count"][q] = len(segments)
+    for k, i in (("seg_dist_min", 0), ("seg_dist_max", 1), ("seg_medium", 2), ("seg_pdf", 3), ("seg_rev_pdf", 3),
+                 ("seg_attenuation", 4)):
+        w[k].extend(s[i] for s in segments)
+    if flags is not None:
+        w["sq_flags"][q] = flags
+
+
+def segment_lists(w):
+    for k in ("seg_dist_min", "seg_dist_max", "seg_pdf", "seg_rev_pdf", "seg_attenuation", "seg_medium"):
+        w[k] = list(w[k])
+
+
+def segment_arrays(w):
+    for k in ("seg_dist_min", "seg_dist_max", "seg_pdf", "seg_rev_pdf"):
+        w[k] = np.asarray(w[k], np.float32)
+    w["seg_attenuation"] = np.asarray(w["seg_attenuation"], np.float32).reshape(-1, 3)
+    w["seg_medium"] = np.asarray(w["seg_medium"], np.int32)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("mode", [engine.MODE_PLAIN, engine.MODE_MIXED], ids=["plain", "mixed"])
+@pytest.mark.parametrize("case", ["infinite_clear_segment", "zero_over_zero"])
+def test_rays_that_end_before_their_neighbours(case, mode):
+    # every other ray has a last segment that passes on no number (exp(-0 inf) in a clear medium, or 0 / 0 of a
+    # SHORT query beam), while its neighbours in the packet have another scattering segment
+    lite = case == "infinite_clear_segment"
+    w = workload(**({} if lite else {"query_beam_type": W.SHORT_BEAM}))
+    segment_lists(w)
+    inside = 0
+    for q in np.nonzero((w["sq_path_length"] == 1) & (w["sq_seg_count"] == 2))[0]:
+        b = int(w["sq_seg_begin"][q])
+        seg = [(w["seg_dist_min"][b + i], w["seg_dist_max"][b + i], int(w["seg_medium"][b + i]), w["seg_pdf"][b + i],
+                w["seg_attenuation"][b + i]) for i in range(2)]
+        assert seg[0][2] == 0 and seg[1][2] == 1
+        t0, t1 = seg[1][0], seg[1][1]
+        flags = int(w["sq_flags"][q]) | W.Q_LITE if lite else int(w["sq_flags"][q]) & ~W.Q_LITE
+        if inside % 2:
+            last = (t1, np.float32(np.inf), 0, 1.0, (1.0, 1.0, 1.0)) if lite else (t1, t1 + 1, 0, 0.0, (0.0, 0.0, 0.0))
+            set_segments(w, q, seg + [last], flags)
+        else:
+            tm = np.float32(0.5) * (t0 + t1)
+            set_segments(w, q, [seg[0], (t0, tm) + seg[1][2:], (tm, t1) + seg[1][2:]], flags)
+        inside += 1
+    assert inside > 50000
+    segment_arrays(w)
+    got, s, want, s0 = both(w, mode)
+    same_pairs(s, s0)
+    assert np.isfinite(want).all() and np.isfinite(got).all()
+    err = G.rel_errors(got.astype(np.float64), want.astype(np.float64))
+    assert err.max() <= (2e-5 if mode == engine.MODE_PLAIN else G.RTOL)
