@@ -67,15 +67,12 @@ __device__ __forceinline__ float axis_k(int k, float x, float y, float z) { retu
 __device__ __forceinline__ float axis_a(int k, float x, float y, float z) { return k == 0 ? y : (k == 1 ? z : x); }
 __device__ __forceinline__ float axis_b(int k, float x, float y, float z) { return k == 0 ? z : (k == 1 ? x : y); }
 
-// Frustum of the rays of the lanes with `valid`; false unless they share their origin exactly, have
-// unit directions (the conservative checks assume them) and advance along one axis.  Warp-wide.
-__device__ __forceinline__ bool packet_frustum(bool valid, V3 o, V3 d, Frustum& F)
+// Frustum of the rays of the lanes with `valid`, along the main axis of a ray (o0, d0); false unless they
+// share its origin exactly, have unit directions (the conservative checks assume them) and advance along
+// that axis.  Warp-wide.  The packet's first ray gives the axis to all its runs of rays: what holds for the
+// packet then holds for each run, whose own first ray may have another main axis.
+__device__ __forceinline__ bool packet_frustum(bool valid, V3 o, V3 d, V3 o0, V3 d0, Frustum& F)
 {
-    const unsigned vote = __ballot_sync(kFull, valid);
-    if (vote == 0u) return false;
-    const int lead = __ffs(vote) - 1;
-    const V3 o0 = v3(__shfl_sync(kFull, o.x, lead), __shfl_sync(kFull, o.y, lead), __shfl_sync(kFull, o.z, lead));
-    const V3 d0 = v3(__shfl_sync(kFull, d.x, lead), __shfl_sync(kFull, d.y, lead), __shfl_sync(kFull, d.z, lead));
     const float ax = fabsf(d0.x), ay = fabsf(d0.y), az = fabsf(d0.z);
     F.o = o0;
     F.k = ax >= ay && ax >= az ? 0 : (ay >= az ? 1 : 2);
@@ -83,7 +80,6 @@ __device__ __forceinline__ bool packet_frustum(bool valid, V3 o, V3 d, Frustum& 
     const float dk = axis_k(F.k, d.x, d.y, d.z) * F.sgn;
     const float len2 = d.x * d.x + d.y * d.y + d.z * d.z;
     const bool ok = o.x == o0.x && o.y == o0.y && o.z == o0.z && dk >= 0.4f && fabsf(len2 - 1.f) <= 2e-6f;
-    if (__any_sync(kFull, valid && !ok)) return false;
     const float sa = axis_a(F.k, d.x, d.y, d.z) / dk, sb = axis_b(F.k, d.x, d.y, d.z) / dk;
     // widened by the rounding of the slopes
     F.a_lo = warp_min(valid ? sa : FLT_MAX) - 2e-6f;
@@ -92,7 +88,7 @@ __device__ __forceinline__ bool packet_frustum(bool valid, V3 o, V3 d, Frustum& 
     F.b_hi = warp_max(valid ? sb : -FLT_MAX) + 2e-6f;
     F.k_lo = warp_min(valid ? dk : FLT_MAX);
     F.k_hi = warp_max(valid ? dk : -FLT_MAX);
-    return true;
+    return !__any_sync(kFull, valid && !ok);
 }
 
 // Whether the frustum between the depths z0 >= 0 and z1 along its axis can meet the box.
@@ -172,7 +168,9 @@ __global__ void __launch_bounds__(256) k_packet_setup(const SegQueriesDev Q, con
         w = cnt_pb2d ? min(__ldg(&cnt_pb2d[q]), 1u << 24) : 0u;
     }
     Frustum F;
-    ok = packet_frustum(valid, o, d, F) && ok;
+    const V3 o0 = v3(__shfl_sync(kFull, o.x, 0), __shfl_sync(kFull, o.y, 0), __shfl_sync(kFull, o.z, 0));
+    const V3 d0 = v3(__shfl_sync(kFull, d.x, 0), __shfl_sync(kFull, d.y, 0), __shfl_sync(kFull, d.z, 0));
+    ok = packet_frustum(valid, o, d, o0, d0, F) && ok;
     ok = __all_sync(kFull, !valid || lo >= 0.f) && ok;
     if (ok) {
         float reach, coord;
@@ -580,8 +578,9 @@ __device__ __forceinline__ void packet_walk(const GatherConsts& K, const BeamBVH
     __syncthreads();
 }
 
-// The packet's rays and frustum, by warp 0 (lane = ray).
-__device__ __forceinline__ void packet_begin(const SegQueriesDev& Q, const int32_t* __restrict__ order, int2 rg,
+// The rays and the frustum of a run rg of a packet's rays, by warp 0 (lane = ray); first: the packet's first
+// ray in the order.
+__device__ __forceinline__ void packet_begin(const SegQueriesDev& Q, const int32_t* __restrict__ order, int first, int2 rg,
                                              const float* __restrict__ bbox, float piece_len, PacketShared& S)
 {
     const int lane = threadIdx.x & 31;
@@ -600,7 +599,9 @@ __device__ __forceinline__ void packet_begin(const SegQueriesDev& Q, const int32
         }
     }
     PacketWalk P;
-    packet_frustum(valid, o, d, P.F);
+    const int64_t q0 = __ldg(&order[first]);
+    packet_frustum(valid, o, d, v3(Q.origin[3 * q0], Q.origin[3 * q0 + 1], Q.origin[3 * q0 + 2]),
+                   v3(Q.direction[3 * q0], Q.direction[3 * q0 + 1], Q.direction[3 * q0 + 2]), P.F);
     packet_scales(P.F.o, bbox, P.reach, P.coord);
     P.near_eps = 4.7e-9f * P.reach * P.reach;
     P.u_eps = 3.5e-5f * P.reach;
@@ -722,7 +723,7 @@ k_bb1d_packet(const __grid_constant__ GatherConsts K, const __grid_constant__ Li
                 const int2 all = range[it & 0xffffffu];
                 const int k = (int)(it >> 24) & 15, log = (int)(it >> 28);
                 const int from = (all.y * k) >> log, to = (all.y * (k + 1)) >> log;
-                packet_begin(Q, order, make_int2(all.x + from, to - from), bbox, piece_len, S);
+                packet_begin(Q, order, all.x, make_int2(all.x + from, to - from), bbox, piece_len, S);
             }
         }
         __syncthreads();

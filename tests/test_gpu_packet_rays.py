@@ -93,3 +93,42 @@ def test_rays_that_end_before_their_neighbours(case, mode):
     assert np.isfinite(want).all() and np.isfinite(got).all()
     err = G.rel_errors(got.astype(np.float64), want.astype(np.float64))
     assert err.max() <= (2e-5 if mode == engine.MODE_PLAIN else G.RTOL)
+
+
+def morton_lanes():
+    """The pixels (x, y) of an 8 x 4 block in the pixel order: bits x0 y0 x1 y1 x2 of the lane."""
+    lane = np.arange(32)
+    return (lane & 1) | (lane >> 1 & 2) | (lane >> 2 & 4), (lane >> 1 & 1) | (lane >> 2 & 2)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("mode", [engine.MODE_PLAIN, engine.MODE_MIXED], ids=["plain", "mixed"])
+def test_wide_fans_of_short_rays(mode):
+    # a dozen pixel blocks hold fans of rays about (1, 1, 1) from one origin; no other query makes a packet
+    # (each has its own origin), so every fan is split into runs of 4 rays.  All advance along the first
+    # ray's main axis x, but the lead of a run has its main axis y, along which its neighbours hardly advance
+    w = workload()
+    rng = np.random.default_rng(3)
+    n = len(w["sq_flags"])
+    w["sq_origin"] += rng.uniform(-1e-3, 1e-3, (n, 3)).astype(np.float32)
+    by_pixel = {int(w["sq_pixel"][q]): q for q in np.nonzero(w["sq_path_length"] == 1)[0]}
+    blocks = [[by_pixel.get((y0 + int(y)) * 419 + x0 + int(x)) for x, y in zip(*morton_lanes())]
+              for y0 in range(0, 316, 4) for x0 in range(0, 416, 8)]
+    blocks = [b for b in blocks if None not in b][::100][:12]
+    segment_lists(w)
+    fans = []
+    for k, block in enumerate(blocks):
+        for lane, q in enumerate(block):
+            d = np.array((0.62, 0.55, 0.56) if lane < 4 else ((0.55, 0.62, 0.56) if lane % 4 == 0 else (0.8, 0.33, 0.5)))
+            d = d + rng.uniform(-0.01, 0.01, 3)
+            w["sq_direction"][q] = d / np.linalg.norm(d)
+            w["sq_origin"][q] = (0.4, 0.45 + 0.002 * k, 0.35)
+            set_segments(w, q, [(0.0, 0.3, 1, 0.9, (0.9, 0.9, 0.9))],
+                         W.Q_ORIGIN_IN_MEDIUM | int(w["sq_flags"][q]))
+            fans.append(q)
+    segment_arrays(w)
+    got, s, want, s0 = both(w, mode)
+    assert s0["count_bb1d"][fans].sum() > 1000
+    same_pairs(s, s0)
+    err = G.rel_errors(got.astype(np.float64), want.astype(np.float64))
+    assert err.max() <= (2e-5 if mode == engine.MODE_PLAIN else G.RTOL)
