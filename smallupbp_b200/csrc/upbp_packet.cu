@@ -220,7 +220,10 @@ struct PacketWalk {
     float dir2_lo, dir2_hi;   // |(slope a, slope b, 1)|^2 over the frustum
     float z0, z1;             // depths of the segment
     // margins of the tests in approximate arithmetic: the squared distance of the lines (a few ulp of
-    // |O2 - O1|) and the beam parameter of their closest points
+    // |O2 - O1|), and the beam parameter of their closest points times 1 - (d.d2)^2.  The latter is a few ulp of
+    // |O2 - O1| too, and 6e-6 of the coordinates: the predicate takes a pair by its own t1, which is off by up to
+    // that (piece_takes_fast), so the lines' closest point may lie that far beyond the ray's end, where the
+    // owner is the piece opposite the end.
     float near_eps, u_eps;
     float reach;              // bound of |O2 - O1|_1
     float coord, scale;       // largest coordinate; that and the end of the segment
@@ -604,7 +607,7 @@ __device__ __forceinline__ void packet_begin(const SegQueriesDev& Q, const int32
                    v3(Q.direction[3 * q0], Q.direction[3 * q0 + 1], Q.direction[3 * q0 + 2]), P.F);
     packet_scales(P.F.o, bbox, P.reach, P.coord);
     P.near_eps = 4.7e-9f * P.reach * P.reach;
-    P.u_eps = 3.5e-5f * P.reach;
+    P.u_eps = 3.5e-5f * P.reach + 6e-6f * P.coord;
     P.piece_len = piece_len;
     const Frustum& F = P.F;
     P.ac = 0.5f * (F.a_lo + F.a_hi), P.ah = 0.5f * (F.a_hi - F.a_lo) + 1e-7f;

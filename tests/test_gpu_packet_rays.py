@@ -132,3 +132,47 @@ def test_wide_fans_of_short_rays(mode):
     same_pairs(s, s0)
     err = G.rel_errors(got.astype(np.float64), want.astype(np.float64))
     assert err.max() <= (2e-5 if mode == engine.MODE_PLAIN else G.RTOL)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("mode", [engine.MODE_PLAIN, engine.MODE_MIXED], ids=["plain", "mixed"])
+def test_segment_ends_at_piece_boundaries_far_from_the_origin(mode):
+    # at coordinates of 4000 the predicate's t1 is off by about 1e-3: it takes pairs whose lines are closest
+    # just beyond the ray's end, and the beam piece that owns such a pair is the one opposite that end, not the
+    # one that holds the lines' closest point.  One beam of three pieces per ray, the end of the middle one close
+    # to both points
+    w = workload()
+    rng = np.random.default_rng(5)
+    for k in ("lv_position", "sq_origin", "pq_position", "beam_origin"):
+        w[k] += np.float32(4000.0)
+    rays = np.nonzero((w["sq_path_length"] == 1) & (w["sq_seg_count"] == 2))[0]
+    n, r, length = len(rays), 0.01, 0.0899
+    o, d = w["sq_origin"][rays].astype(np.float64), w["sq_direction"][rays].astype(np.float64)
+    last = w["sq_seg_begin"][rays] + 1
+    t0, t1 = w["seg_dist_min"][last], w["seg_dist_max"][last]
+    t = t0 + (t1 - t0) * rng.uniform(0.3, 0.9, n)
+    # directions at 30 to 60 degrees from the ray's
+    c = rng.uniform(0.5, 0.87, n)
+    v = np.cross(d, rng.normal(size=(n, 3)))
+    v /= np.linalg.norm(v, axis=1, keepdims=True)
+    d2 = (c[:, None] * d + np.sqrt(1 - c * c)[:, None] * v)
+    d2 = (d2 / np.linalg.norm(d2, axis=1, keepdims=True)).astype(np.float32)
+    side = np.cross(d, d2)
+    side /= np.linalg.norm(side, axis=1, keepdims=True)
+    u = length * 2 / 3 + rng.uniform(-1e-3, 1e-3, n)
+    o2 = (o + t[:, None] * d + 0.3 * r * side - u[:, None] * d2.astype(np.float64)).astype(np.float32)
+    # the lines' closest point for the rounded inputs, and the rays' ends just before it
+    b64, w64 = d2.astype(np.float64), o - o2.astype(np.float64)
+    aa, cc, bb = (d * d).sum(1), (b64 * b64).sum(1), (d * b64).sum(1)
+    dd, ee = (d * w64).sum(1), (b64 * w64).sum(1)
+    t = (bb * ee - cc * dd) / (aa * cc - bb * bb)
+    w["seg_dist_max"][last] = t - rng.uniform(0.0, 1e-3, n)
+    old = len(w["beam_length"])
+    for k in [k for k in w if k.startswith("beam_")]:
+        w[k] = w[k][np.arange(n) % old].copy()
+    w["beam_origin"], w["beam_direction"] = o2, d2
+    w["beam_length"][:] = length
+    w["beam_medium_id"][:] = 1
+    got, s, want, s0 = both(w, mode, beam_piece_radii=3.0)
+    assert s0["count_bb1d"][rays].sum() > n // 10
+    same_pairs(s, s0)
