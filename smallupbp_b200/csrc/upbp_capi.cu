@@ -984,33 +984,34 @@ gen::GenLaunch generic_launch(upbp_ctx* c, const CamSum* cs_seg, const CamSum* c
 PacketsDev find_packets(upbp_ctx* c, const SegQueriesDev& Q, const int32_t* order, const uint32_t* counts,
                         float piece_len, int resident, cudaStream_t s)
 {
-    const int n = packet_blocks(c->P.image_width, c->P.image_height), slots = n * kPacketParts;
+    const int n = packet_max(c->P.image_width, c->P.image_height, Q.n), slots = packet_slots(n, resident);
     ensure(c, c->pk_range, sizeof(int2) * n);
     ensure(c, c->pk_weight, sizeof(uint32_t) * n);
     ensure(c, c->pk_key, sizeof(uint32_t) * slots);
     ensure(c, c->pk_key_sorted, sizeof(uint32_t) * slots);
-    ensure(c, c->pk_item, sizeof(uint32_t) * slots);
-    ensure(c, c->pk_item_sorted, sizeof(uint32_t) * slots);
+    ensure(c, c->pk_item, sizeof(unsigned long long) * slots);
+    ensure(c, c->pk_item_sorted, sizeof(unsigned long long) * slots);
     ensure(c, c->pk_in, (size_t)Q.n);
     ensure(c, c->pk_totals, sizeof(PacketTotals));
     ck(c, cudaMemsetAsync(c->pk_in.p, 0, (size_t)Q.n, s), "memset");
+    ck(c, cudaMemsetAsync(c->pk_key.p, 0, sizeof(uint32_t) * slots, s), "memset");
     ck(c, cudaMemsetAsync(c->pk_totals.p, 0, sizeof(PacketTotals), s), "memset");
     PacketsDev P{};
     P.range = c->pk_range.as<int2>();
     P.weight = c->pk_weight.as<uint32_t>();
     P.key = c->pk_key.as<uint32_t>();
-    P.item = c->pk_item.as<uint32_t>();
-    P.item_sorted = c->pk_item_sorted.as<uint32_t>();
+    P.item = c->pk_item.as<unsigned long long>();
+    P.item_sorted = c->pk_item_sorted.as<unsigned long long>();
     P.in_packet = c->pk_in.as<uint8_t>();
     P.totals = c->pk_totals.as<PacketTotals>();
-    launch_packet_setup(Q, c->q_keys_sorted.as<uint32_t>(), order, counts, c->P.image_width, c->P.image_height,
-                        c->bbox_pc.as<float>(), piece_len, resident, P, s);
+    launch_packet_setup(Q, c->q_keys_sorted.as<uint32_t>(), order, counts, n,
+                        (int64_t)c->P.image_width * c->P.image_height, c->bbox_pc.as<float>(), piece_len, resident, P, s);
     size_t b = 0;
     cub::DeviceRadixSort::SortPairsDescending(nullptr, b, P.key, c->pk_key_sorted.as<uint32_t>(), P.item,
-                                              c->pk_item_sorted.as<uint32_t>(), slots, 0, 32, s);
+                                              c->pk_item_sorted.as<unsigned long long>(), slots, 0, 32, s);
     ensure(c, c->cub_tmp, b);
     ck(c, cub::DeviceRadixSort::SortPairsDescending(c->cub_tmp.p, b, P.key, c->pk_key_sorted.as<uint32_t>(), P.item,
-                                                    c->pk_item_sorted.as<uint32_t>(), slots, 0, 32, s),
+                                                    c->pk_item_sorted.as<unsigned long long>(), slots, 0, 32, s),
        "SortPairsDescending");
     c->eval_launches += 6;
     return P;
@@ -1141,12 +1142,9 @@ void do_evaluate(upbp_ctx* c)
     const int32_t* bb_order = order;
     const bool counts = (c->P.techniques & UPBP_PB2D) && c->n_ph > 0;
     // Camera rays in packets: they need the pixel order (its key holds 14 bits per axis), pieces, and
-    // enough packets to keep the blocks busy to the end: against one warp per query the packets take
-    // 0.6-0.8 of the time at 400 thousand queries and more, 0.7-1.0 at 100 thousand, and 1.0-1.3 below
-    // 70 thousand (cube, boxes and KNN scenes, measured either way).
-    constexpr int64_t kPacketQueries = 100000;
+    // enough camera queries (kPacketCamera), which the setup kernel counts.
     const bool packets = order && c->query_order == 1 && !fused && !grid_mode && c->bb1d_kernel >= 1 &&
-                         nq >= kPacketQueries && c->n_pieces > 0 && npix > 0 && c->P.image_width <= (1 << 14) &&
+                         nq >= (int64_t)kPacketCamera && c->n_pieces > 0 && npix > 0 && c->P.image_width <= (1 << 14) &&
                          c->P.image_height <= (1 << 14);
     const float piece_len = std::max(1e-6f, c->piece_len_r * c->P.radius_bb1d);
     const int packet_grid = packets ? c->num_sms * bb1d_packet_blocks_per_sm(mixed) : 0;
@@ -1162,8 +1160,8 @@ void do_evaluate(upbp_ctx* c)
         ensure(c, c->bb_sum, sizeof(unsigned long long));
         ck(c, cudaMemsetAsync(c->bb_sum.p, 0, sizeof(unsigned long long), s), "memset");
         launch_heavy_keys(counts ? c->cnt_pb2d.as<uint32_t>() : nullptr, nq, c->bb_sum.as<unsigned long long>(),
-                          kHeavyFactor, c->q_keys.as<uint32_t>(), PK.in_packet, c->bb_keys.as<uint32_t>(),
-                          c->bb_iota.as<int32_t>(), s);
+                          kHeavyFactor, c->q_keys.as<uint32_t>(), PK.in_packet,
+                          packets ? &PK.totals->queries : nullptr, c->bb_keys.as<uint32_t>(), c->bb_iota.as<int32_t>(), s);
         size_t b = 0;
         cub::DeviceRadixSort::SortPairs(nullptr, b, c->bb_keys.as<uint32_t>(), c->bb_keys_sorted.as<uint32_t>(),
                                         c->bb_iota.as<int32_t>(), c->bb_order.as<int32_t>(), (int)nq, 0, 32, s);

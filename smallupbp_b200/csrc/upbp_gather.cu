@@ -1400,26 +1400,28 @@ __global__ void k_sum_counts(const uint32_t* __restrict__ cnt, int64_t n, unsign
 
 // BB1D work order: the queries whose PB2D candidate count exceeds `factor` times the mean come
 // first (they are the heaviest BB1D queries too), each group in Morton order of the midpoints.
-// Without counts (cnt NULL) none is heavy.  The queries that packets hold (in_packet, or NULL) go last.
+// Without counts (cnt NULL) none is heavy.  The queries that packets hold (in_packet, or NULL; none where
+// *held is 0) go last.
 __global__ void k_heavy_keys(const uint32_t* __restrict__ cnt, int64_t n, const unsigned long long* __restrict__ sum,
                              unsigned factor, const uint32_t* __restrict__ morton,
-                             const uint8_t* __restrict__ in_packet, uint32_t* keys, int32_t* iota)
+                             const uint8_t* __restrict__ in_packet, const unsigned* __restrict__ held, uint32_t* keys,
+                             int32_t* iota)
 {
     const int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (q >= n) return;
     const bool heavy = cnt && (unsigned long long)cnt[q] * (unsigned long long)n > (unsigned long long)factor * *sum;
-    keys[q] = in_packet && in_packet[q] ? 0xffffffffu : (heavy ? 0u : (1u << 30)) | morton[q];
+    keys[q] = in_packet && in_packet[q] && *held ? 0xffffffffu : (heavy ? 0u : (1u << 30)) | morton[q];
     iota[q] = (int32_t)q;
 }
 }  // namespace
 
 void launch_heavy_keys(const uint32_t* cnt, int64_t n, unsigned long long* sum, unsigned factor,
-                       const uint32_t* morton, const uint8_t* in_packet, uint32_t* keys, int32_t* iota,
-                       cudaStream_t stream)
+                       const uint32_t* morton, const uint8_t* in_packet, const unsigned* held, uint32_t* keys,
+                       int32_t* iota, cudaStream_t stream)
 {
     if (n <= 0) return;
     if (cnt) k_sum_counts<<<148 * 4, 256, 0, stream>>>(cnt, n, sum);
-    k_heavy_keys<<<(int)((n + 255) / 256), 256, 0, stream>>>(cnt, n, sum, factor, morton, in_packet, keys, iota);
+    k_heavy_keys<<<(int)((n + 255) / 256), 256, 0, stream>>>(cnt, n, sum, factor, morton, in_packet, held, keys, iota);
 }
 
 void launch_beam_payload(int n, const float4* bm_thr, const float4* bm_pdf, const int2* bm_link, const float* bm_radius,

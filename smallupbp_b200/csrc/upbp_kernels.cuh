@@ -249,8 +249,8 @@ void launch_query_keys(const SegQueriesDev& Q, const float* bbox, int mode, int 
 // without counts), each group in the given Morton order, and those that packets hold last; *sum
 // must be zero on entry
 void launch_heavy_keys(const uint32_t* cnt, int64_t n, unsigned long long* sum, unsigned factor,
-                       const uint32_t* morton, const uint8_t* in_packet, uint32_t* keys, int32_t* iota,
-                       cudaStream_t stream);
+                       const uint32_t* morton, const uint8_t* in_packet, const unsigned* held, uint32_t* keys,
+                       int32_t* iota, cudaStream_t stream);
 int bb1d_warp_blocks_per_sm(bool mixed, int variant);
 int pb2d_warp_blocks_per_sm(bool mixed);
 void launch_pb2d_warp(const GatherConsts& K, const LightSoA& L, const PhotonBVH& P, const SegQueriesDev& Q,

@@ -20,6 +20,7 @@
 // The candidate set is the one of the per-query kernels: every accepted pair passes the reference's FP32
 // predicate (PhotonBeam.hxx:238-296), the radius test and the reach rule (upbp_device.cuh); the checks
 // before them are conservative.
+#include <algorithm>
 #include <cfloat>
 #include <cstdint>
 
@@ -31,6 +32,7 @@ namespace upbp {
 namespace {
 
 constexpr float kNan = __builtin_nanf("");
+constexpr float kPacketShare = 0.6f;        // k_packet_items
 constexpr int kPWarps = 8;                  // warps per block
 constexpr int kPThreads = kPWarps * 32;
 // The frustum walk pops up to kPNodes nodes a step, two threads per node (one per child).  Its stack
@@ -67,19 +69,27 @@ __device__ __forceinline__ float axis_k(int k, float x, float y, float z) { retu
 __device__ __forceinline__ float axis_a(int k, float x, float y, float z) { return k == 0 ? y : (k == 1 ? z : x); }
 __device__ __forceinline__ float axis_b(int k, float x, float y, float z) { return k == 0 ? z : (k == 1 ? x : y); }
 
-// Frustum of the rays of the lanes with `valid`, along the main axis of a ray (o0, d0); false unless they
-// share its origin exactly, have unit directions (the conservative checks assume them) and advance along
-// that axis.  Warp-wide.  The packet's first ray gives the axis to all its runs of rays: what holds for the
-// packet then holds for each run, whose own first ray may have another main axis.
-__device__ __forceinline__ bool packet_frustum(bool valid, V3 o, V3 d, V3 o0, V3 d0, Frustum& F)
+// The main axis of a direction: k << 1, and 1 for the negative sense.
+__device__ __forceinline__ int main_axis(V3 d)
 {
-    const float ax = fabsf(d0.x), ay = fabsf(d0.y), az = fabsf(d0.z);
+    const float ax = fabsf(d.x), ay = fabsf(d.y), az = fabsf(d.z);
+    const int k = ax >= ay && ax >= az ? 0 : (ay >= az ? 1 : 2);
+    return k << 1 | (axis_k(k, d.x, d.y, d.z) < 0.f ? 1 : 0);
+}
+
+// Frustum along `axis` (main_axis) of the rays of the lanes with `valid`, which share the origin o0; false unless
+// they have it exactly, have unit directions (the conservative checks assume them) and advance along the axis.
+// Warp-wide.  The packet's first ray gives the axis to all of its runs of rays: what holds for the packet then
+// holds for each run, whose own first ray may have another main axis.
+__device__ __forceinline__ bool packet_frustum(bool valid, V3 o, V3 d, V3 o0, int axis, Frustum& F)
+{
     F.o = o0;
-    F.k = ax >= ay && ax >= az ? 0 : (ay >= az ? 1 : 2);
-    F.sgn = axis_k(F.k, d0.x, d0.y, d0.z) < 0.f ? -1.f : 1.f;
+    F.k = axis >> 1;
+    F.sgn = axis & 1 ? -1.f : 1.f;
     const float dk = axis_k(F.k, d.x, d.y, d.z) * F.sgn;
     const float len2 = d.x * d.x + d.y * d.y + d.z * d.z;
     const bool ok = o.x == o0.x && o.y == o0.y && o.z == o0.z && dk >= 0.4f && fabsf(len2 - 1.f) <= 2e-6f;
+    if (__any_sync(kFull, valid && !ok)) return false;
     const float sa = axis_a(F.k, d.x, d.y, d.z) / dk, sb = axis_b(F.k, d.x, d.y, d.z) / dk;
     // widened by the rounding of the slopes
     F.a_lo = warp_min(valid ? sa : FLT_MAX) - 2e-6f;
@@ -88,7 +98,13 @@ __device__ __forceinline__ bool packet_frustum(bool valid, V3 o, V3 d, V3 o0, V3
     F.b_hi = warp_max(valid ? sb : -FLT_MAX) + 2e-6f;
     F.k_lo = warp_min(valid ? dk : FLT_MAX);
     F.k_hi = warp_max(valid ? dk : -FLT_MAX);
-    return !__any_sync(kFull, valid && !ok);
+    return true;
+}
+
+// A work item: the first ray of the run in the order, how many, and the axis of the packet.
+__device__ __forceinline__ unsigned long long packet_item(int first, int count, int axis)
+{
+    return (unsigned long long)(unsigned)first | (unsigned long long)(count | axis << 8) << 32;
 }
 
 // Whether the frustum between the depths z0 >= 0 and z1 along its axis can meet the box.
@@ -116,74 +132,70 @@ __device__ __forceinline__ void packet_scales(V3 o, const float* __restrict__ bb
 }
 
 // ----------------------------------------------------------------- packets of an image
-__device__ __forceinline__ uint32_t spread2(uint32_t v)
-{
-    uint32_t r = 0;
-    for (int b = 0; b < 14; ++b) r |= ((v >> b) & 1u) << (2 * b);
-    return r;
-}
-
-__device__ __forceinline__ int lower_bound(const uint32_t* __restrict__ keys, int n, uint32_t v)
-{
-    int lo = 0, hi = n;
-    while (lo < hi) {
-        const int mid = (lo + hi) >> 1;
-        if (__ldg(&keys[mid]) < v) lo = mid + 1;
-        else hi = mid;
-    }
-    return lo;
-}
-
-// One warp per 8 x 4 pixel block: its queries are consecutive in the pixel order (the sort key's low
-// five bits count the pixels of an aligned block).  They form a packet if there are at most 32 of
-// them, their rays make a frustum, and that is at most max_width across at its far end: the rays of a
-// frustum much wider than the beam pieces share few of them.
-// weight: the work estimate (PB2D candidates), 0 for a block without a packet.
+// The pixel blocks (8 x 4) of the queries: a block's camera rays are consecutive in the pixel order, whose keys'
+// low five bits count the pixels of an aligned block (the other segments' keys have bit 29).  A warp takes the
+// blocks that begin at its 32 places of the order, one after the other, so the work grows with the
+// queries, not with the image.  A block's rays form a packet if there are at most 32 of them, they make a
+// frustum, and that is at most max_width across at its far end: the rays of a frustum much wider than the beam
+// pieces share few of them.  The packets are listed in no particular order.
 __global__ void __launch_bounds__(256) k_packet_setup(const SegQueriesDev Q, const uint32_t* __restrict__ keys,
                                                       const int32_t* __restrict__ order,
-                                                      const uint32_t* __restrict__ cnt_pb2d, int width, int height,
-                                                      const float* __restrict__ bbox, float max_width, int2* range,
-                                                      uint32_t* weight, uint8_t* in_packet, PacketTotals* totals)
+                                                      const uint32_t* __restrict__ cnt_pb2d,
+                                                      int64_t n_pixels, const float* __restrict__ bbox, float max_width,
+                                                      int2* range, uint32_t* weight, uint8_t* in_packet,
+                                                      PacketTotals* totals)
 {
-    const int bw = (width + 7) / 8, bh = (height + 3) / 4;
-    const int b = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
-    if (b >= bw * bh) return;
-    const uint32_t code = spread2((uint32_t)(b % bw) * 8u) | (spread2((uint32_t)(b / bw) * 4u) << 1);
-    const int mine = lane < 2 ? lower_bound(keys, (int)Q.n, code + 32u * (uint32_t)lane) : 0;
-    const int start = __shfl_sync(kFull, mine, 0), count = __shfl_sync(kFull, mine, 1) - start;
-    bool ok = count > 0 && count <= 32;
-    const bool valid = ok && lane < count;
-    const int64_t q = valid ? (int64_t)__ldg(&order[start + lane]) : 0;
-    V3 o = v3(0.f, 0.f, 0.f), d = o;
-    float lo = FLT_MAX, hi = 0.f;
-    unsigned w = 0;
-    if (valid) {
-        o = v3(Q.origin[3 * q], Q.origin[3 * q + 1], Q.origin[3 * q + 2]);
-        d = v3(Q.direction[3 * q], Q.direction[3 * q + 1], Q.direction[3 * q + 2]);
-        const int sb = Q.seg_begin[q], sc = Q.seg_count[q];
-        for (int i = 0; i < sc; ++i) {
-            lo = fminf(lo, Q.seg_dist_min[sb + i]);
-            hi = fmaxf(hi, Q.seg_dist_max[sb + i]);
+    constexpr uint32_t kNoBlock = 0xffffffffu;
+    const int n = (int)Q.n;
+    const int base = (int)((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) & ~31ll), lane = threadIdx.x & 31;
+    if (base >= n) return;
+    const auto block_of = [&](int i) {
+        const uint32_t k = i < n ? __ldg(&keys[i]) : kNoBlock;
+        return k < (1u << 28) ? k >> 5 : kNoBlock;
+    };
+    const int i = base + lane;
+    const uint32_t mine = block_of(i), before = i > 0 ? block_of(i - 1) : kNoBlock;
+    if (mine != kNoBlock && block_of(i + 1) == kNoBlock) totals->camera = (unsigned)i + 1u;
+    unsigned starts = __ballot_sync(kFull, mine != kNoBlock && mine != before);
+    for (; starts; starts &= starts - 1) {
+        const int from = __ffs(starts) - 1, start = base + from;
+        const uint32_t block = __shfl_sync(kFull, mine, from);
+        const unsigned members = __ballot_sync(kFull, block_of(start + lane) == block);
+        const int count = __popc(members);
+        bool ok = !(count == 32 && block_of(start + 32) == block);
+        const bool valid = lane < count;
+        const int64_t q = valid ? (int64_t)__ldg(&order[start + lane]) : 0;
+        V3 o = v3(0.f, 0.f, 0.f), d = o;
+        float lo = FLT_MAX, hi = 0.f;
+        unsigned w = 0;
+        if (valid && ok) {
+            o = v3(Q.origin[3 * q], Q.origin[3 * q + 1], Q.origin[3 * q + 2]);
+            d = v3(Q.direction[3 * q], Q.direction[3 * q + 1], Q.direction[3 * q + 2]);
+            const int sb = Q.seg_begin[q], sc = Q.seg_count[q];
+            for (int k = 0; k < sc; ++k) {
+                lo = fminf(lo, Q.seg_dist_min[sb + k]);
+                hi = fmaxf(hi, Q.seg_dist_max[sb + k]);
+            }
+            w = cnt_pb2d ? min(__ldg(&cnt_pb2d[q]), 1u << 24) : 0u;
         }
-        w = cnt_pb2d ? min(__ldg(&cnt_pb2d[q]), 1u << 24) : 0u;
-    }
-    Frustum F;
-    const V3 o0 = v3(__shfl_sync(kFull, o.x, 0), __shfl_sync(kFull, o.y, 0), __shfl_sync(kFull, o.z, 0));
-    const V3 d0 = v3(__shfl_sync(kFull, d.x, 0), __shfl_sync(kFull, d.y, 0), __shfl_sync(kFull, d.z, 0));
-    ok = packet_frustum(valid, o, d, o0, d0, F) && ok;
-    ok = __all_sync(kFull, !valid || lo >= 0.f) && ok;
-    if (ok) {
-        float reach, coord;
-        packet_scales(F.o, bbox, reach, coord);
-        ok = fmaxf(F.a_hi - F.a_lo, F.b_hi - F.b_lo) * fminf(warp_max(hi), reach) <= max_width;
-    }
-    w = __reduce_add_sync(kFull, w);
-    if (ok && valid) in_packet[q] = 1;
-    if (lane == 0) {
-        range[b] = make_int2(start, count);
-        weight[b] = ok ? w + 1u : 0u;
+        Frustum F;
+        const V3 o0 = v3(__shfl_sync(kFull, o.x, 0), __shfl_sync(kFull, o.y, 0), __shfl_sync(kFull, o.z, 0));
+        const int axis = __shfl_sync(kFull, main_axis(d), 0);
+        ok = packet_frustum(valid, o, d, o0, axis, F) && ok;
+        ok = __all_sync(kFull, !valid || (lo >= 0.f && Q.pixel[q] < n_pixels)) && ok;
         if (ok) {
-            atomicAdd(&totals->queries, (unsigned)count);
+            float reach, coord;
+            packet_scales(F.o, bbox, reach, coord);
+            ok = fmaxf(F.a_hi - F.a_lo, F.b_hi - F.b_lo) * fminf(warp_max(hi), reach) <= max_width;
+        }
+        w = __reduce_add_sync(kFull, w);
+        if (!ok) continue;
+        if (valid) in_packet[q] = 1;
+        if (lane == 0) {
+            const unsigned p = atomicAdd(&totals->packets, 1u);
+            range[p] = make_int2(start, count | axis << 8);
+            weight[p] = w + 1u;  // the work estimate (PB2D candidates)
+            atomicAdd(&totals->rays, (unsigned)count);
             atomicAdd(&totals->weight, (unsigned long long)w + 1ull);
         }
     }
@@ -193,21 +205,28 @@ __global__ void __launch_bounds__(256) k_packet_setup(const SegQueriesDev Q, con
 // all work (the heaviest packet has 15 times the mean's work, and in a small image a packet's block
 // would run long after the others are done).  Each item is a packet of its own, with a narrower frustum,
 // but walks the tree again: at cube512 a share of 0.05 / 0.25 / 0.6 / 1 of what a resident block gets
-// on average took 18.4 / 15.7 / 14.9 / 15.0 ms.  The items are sorted by weight; slots without one have 0.
+// on average took 18.4 / 15.7 / 14.9 / 15.0 ms.  The items are sorted by weight; slots without one have 0 (the
+// caller's).  A packet of P parts has more than share P / 2 of the weight, so that there are at most
+// 2 / share items more than packets.
 __global__ void __launch_bounds__(256) k_packet_items(const uint32_t* __restrict__ weight, const int2* __restrict__ range,
-                                                      int n, float share, PacketTotals* totals, uint32_t* key,
-                                                      uint32_t* item)
+                                                      float share, unsigned slots, PacketTotals* totals, uint32_t* key,
+                                                      unsigned long long* item)
 {
-    const int b = blockIdx.x * blockDim.x + threadIdx.x;
-    if (b >= n) return;
-    const uint32_t w = weight[b];
+    const unsigned p = blockIdx.x * blockDim.x + threadIdx.x;
+    if (p >= totals->packets || totals->camera < kPacketCamera) return;
+    if (p == 0) totals->queries = totals->rays;
+    const uint32_t w = weight[p];
+    const int2 r = range[p];
+    const int count = r.y & 0xff;
     const float limit = share * (float)totals->weight;
-    int parts = 1;
-    while (parts < kPacketParts && (float)w > limit * (float)parts && parts < range[b].y) parts *= 2;
-    if (w) atomicAdd(&totals->items, (unsigned)parts);
-    for (int k = 0; k < kPacketParts; ++k) {
-        key[b * kPacketParts + k] = w && k < parts ? max(1u, w / (uint32_t)parts) : 0u;
-        item[b * kPacketParts + k] = (uint32_t)b | ((uint32_t)k << 24) | ((uint32_t)(__ffs(parts) - 1) << 28);
+    int log = 0;
+    while (1 << log < kPacketParts && (float)w > limit * (float)(1 << log) && 2 << log <= count) ++log;
+    const unsigned at = atomicAdd(&totals->items, 1u << log);
+    for (int k = 0; k < 1 << log; ++k) {
+        const int from = (count * k) >> log, to = (count * (k + 1)) >> log;
+        if (at + k >= slots) return;  // cannot happen (see above); kept as a guard
+        key[at + k] = max(1u, w >> log);
+        item[at + k] = packet_item(r.x + from, to - from, r.y >> 8);
     }
 }
 
@@ -581,9 +600,8 @@ __device__ __forceinline__ void packet_walk(const GatherConsts& K, const BeamBVH
     __syncthreads();
 }
 
-// The rays and the frustum of a run rg of a packet's rays, by warp 0 (lane = ray); first: the packet's first
-// ray in the order.
-__device__ __forceinline__ void packet_begin(const SegQueriesDev& Q, const int32_t* __restrict__ order, int first, int2 rg,
+// The rays and the frustum (along `axis`) of a run rg of a packet's rays, by warp 0 (lane = ray).
+__device__ __forceinline__ void packet_begin(const SegQueriesDev& Q, const int32_t* __restrict__ order, int2 rg, int axis,
                                              const float* __restrict__ bbox, float piece_len, PacketShared& S)
 {
     const int lane = threadIdx.x & 31;
@@ -602,9 +620,8 @@ __device__ __forceinline__ void packet_begin(const SegQueriesDev& Q, const int32
         }
     }
     PacketWalk P;
-    const int64_t q0 = __ldg(&order[first]);
-    packet_frustum(valid, o, d, v3(Q.origin[3 * q0], Q.origin[3 * q0 + 1], Q.origin[3 * q0 + 2]),
-                   v3(Q.direction[3 * q0], Q.direction[3 * q0 + 1], Q.direction[3 * q0 + 2]), P.F);
+    const V3 o0 = v3(__shfl_sync(kFull, o.x, 0), __shfl_sync(kFull, o.y, 0), __shfl_sync(kFull, o.z, 0));
+    packet_frustum(valid, o, d, o0, axis, P.F);
     packet_scales(P.F.o, bbox, P.reach, P.coord);
     P.near_eps = 4.7e-9f * P.reach * P.reach;
     P.u_eps = 3.5e-5f * P.reach + 6e-6f * P.coord;
@@ -709,8 +726,8 @@ template <bool kMixed, int kMinBlocks>
 __global__ void __launch_bounds__(kPThreads, kMinBlocks)
 k_bb1d_packet(const __grid_constant__ GatherConsts K, const __grid_constant__ LightSoA Lv,
               const __grid_constant__ BeamBVH B, const __grid_constant__ BeamSoA Bs, const SegQueriesDev Q,
-              const Outputs O, const int32_t* __restrict__ order, const int2* __restrict__ range,
-              const uint32_t* __restrict__ items, const PacketTotals* __restrict__ totals,
+              const Outputs O, const int32_t* __restrict__ order, const unsigned long long* __restrict__ items,
+              const PacketTotals* __restrict__ totals,
               const float* __restrict__ bbox, float piece_len, unsigned* work)
 {
     extern __shared__ __align__(16) unsigned char smem[];
@@ -722,11 +739,9 @@ k_bb1d_packet(const __grid_constant__ GatherConsts K, const __grid_constant__ Li
             if (lane == 0) S.next = atomicAdd(work, 1u);
             __syncwarp();
             if (S.next < totals->items) {
-                const uint32_t it = items[S.next];
-                const int2 all = range[it & 0xffffffu];
-                const int k = (int)(it >> 24) & 15, log = (int)(it >> 28);
-                const int from = (all.y * k) >> log, to = (all.y * (k + 1)) >> log;
-                packet_begin(Q, order, all.x, make_int2(all.x + from, to - from), bbox, piece_len, S);
+                const unsigned long long it = items[S.next];
+                packet_begin(Q, order, make_int2((int)(unsigned)it, (int)(it >> 32) & 0xff), (int)(it >> 40), bbox, piece_len,
+                             S);
             }
         }
         __syncthreads();
@@ -797,18 +812,23 @@ int blocks_per_sm()
 
 }  // namespace
 
-int packet_blocks(int width, int height) { return ((width + 7) / 8) * ((height + 3) / 4); }
+int packet_max(int width, int height, int64_t n)
+{
+    return (int)std::min<int64_t>((int64_t)((width + 7) / 8) * ((height + 3) / 4), n);
+}
+int packet_slots(int packets, int resident) { return packets + (int)(2.f / kPacketShare) * resident + 2 * resident; }
 
 void launch_packet_setup(const SegQueriesDev& Q, const uint32_t* keys, const int32_t* order, const uint32_t* cnt_pb2d,
-                         int width, int height, const float* bbox, float piece_len, int resident, const PacketsDev& P,
-                         cudaStream_t s)
+                         int packets, int64_t n_pixels, const float* bbox, float piece_len, int resident,
+                         const PacketsDev& P, cudaStream_t s)
 {
-    const int n = packet_blocks(width, height);
     // the widest packet, in piece lengths
     constexpr float kPacketWidth = 4.f;
-    k_packet_setup<<<(n + 7) / 8, 256, 0, s>>>(Q, keys, order, cnt_pb2d, width, height, bbox, kPacketWidth * piece_len,
-                                               P.range, P.weight, P.in_packet, P.totals);
-    k_packet_items<<<(n + 255) / 256, 256, 0, s>>>(P.weight, P.range, n, 0.6f / (float)resident, P.totals, P.key, P.item);
+    k_packet_setup<<<(unsigned)((Q.n + 255) / 256), 256, 0, s>>>(Q, keys, order, cnt_pb2d, n_pixels, bbox,
+                                                                 kPacketWidth * piece_len, P.range, P.weight, P.in_packet,
+                                                                 P.totals);
+    k_packet_items<<<(packets + 255) / 256, 256, 0, s>>>(P.weight, P.range, kPacketShare / (float)resident,
+                                                         (unsigned)packet_slots(packets, resident), P.totals, P.key, P.item);
 }
 
 int bb1d_packet_blocks_per_sm(bool mixed) { return mixed ? blocks_per_sm<true>() : blocks_per_sm<false>(); }
@@ -820,10 +840,10 @@ void launch_bb1d_packet(const GatherConsts& K, const LightSoA& L, const BeamBVH&
     const int bytes = (int)sizeof(PacketShared);
     if (mixed)
         k_bb1d_packet<true, kPBlocks><<<grid, kPThreads, bytes, s>>>(
-            K, L, B, S, Q, O, order, P.range, P.item_sorted, P.totals, bbox, piece_len, work);
+            K, L, B, S, Q, O, order, P.item_sorted, P.totals, bbox, piece_len, work);
     else
         k_bb1d_packet<false, kPBlocks><<<grid, kPThreads, bytes, s>>>(
-            K, L, B, S, Q, O, order, P.range, P.item_sorted, P.totals, bbox, piece_len, work);
+            K, L, B, S, Q, O, order, P.item_sorted, P.totals, bbox, piece_len, work);
 }
 
 }  // namespace upbp

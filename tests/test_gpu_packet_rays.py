@@ -176,3 +176,36 @@ def test_segment_ends_at_piece_boundaries_far_from_the_origin(mode):
     got, s, want, s0 = both(w, mode, beam_piece_radii=3.0)
     assert s0["count_bb1d"][rays].sum() > n // 10
     same_pairs(s, s0)
+
+
+@pytest.mark.gpu
+def test_few_camera_queries_among_many_make_no_packets():
+    # 40,000 camera queries on a pixel among 138,000 segment queries: too few to keep the packets' blocks busy
+    w = workload()
+    first = np.nonzero(w["sq_path_length"] == 1)[0]
+    w["sq_pixel"][first[40000:]] = -1
+    _, s, tested = results(w, engine.MODE_MIXED, query_order=1)
+    _, s0, tested0 = results(w, engine.MODE_MIXED, query_order=0)
+    assert tested == tested0
+    same_pairs(s, s0)
+
+
+@pytest.mark.gpu
+def test_packets_of_a_crop_take_memory_by_the_queries():
+    # the queries of 419 x 317 pixels in an image of 8192 x 8192: the packets' lists, at most 100 bytes per query
+    w = workload()
+    x, y = w["sq_pixel"] % 419, w["sq_pixel"] // 419
+    w["sq_pixel"] = np.where(w["sq_pixel"] < 0, -1, (y + 4000) * 8192 + x + 4001).astype(np.int32)
+    w["pq_pixel"][:] = -1
+    w["params"]["image_width"], w["params"]["image_height"] = 8192, 8192
+    made = []
+    for order in (0, 1):
+        with engine.EstimatorStage(0, engine.MODE_PLAIN) as st:
+            st.set_tuning(query_order=order)
+            st.run(w)
+            made.append((st.device_bytes(), st.query_stats(), st.tested_counts()["bb1d"], st.segment_results()[1]))
+    (bytes0, s0, tested0, want), (bytes1, s, tested, got) = made
+    assert tested != tested0  # the packets ran
+    same_pairs(s, s0)
+    assert G.rel_errors(got.astype(np.float64), want.astype(np.float64)).max() <= 2e-5
+    assert bytes1 - bytes0 <= 100 * len(w["sq_pixel"])
