@@ -336,14 +336,13 @@ __device__ Rgb bb1d_contrib(const GatherConsts& K, const DMedium& m, const Light
 
 // PhotonBeam::accumulate2 (mixed mode) with the beam's payload packed per piece, at the lines' closest
 // approach g.  kDirect: a camera path of length 1 (s.L is not read), which has no MIS records before the
-// merged vertex.  Fewer divisions, the others as reciprocals of the special function unit: one factor for the
-// three channels, and the beam's side of the weight arranged so that neither the squared distance D nor the
-// reverse pdf R along the beam is divided by:
-//   wLight = last * pdfAInv * (D bptb + phase * cont * cos * (d R + e)) / rspB.
-// (No constant is inverted beforehand: its rounding would be the same in every pair.)
-// BB1D against the version with a division per term, without packets: nested boxes with 300 x 300 pixels 4.74 ->
-// 4.49 ms, LONG beams with 256 x 200 pixels 2.98 -> 2.82 ms; per-query error against FP64 at cube512 p50
-// 2.56e-7 -> 2.58e-7, root mean square 1.325e-6 in both.
+// merged vertex.  The general form's operations, but for the beam's side of the weight, arranged so that neither
+// the squared distance D nor the reverse pdf R along the beam is divided by:
+//   wLight = last * pdfAInv * (D bptb + phase * cont * cos * (d R + e)) / rspB
+// (cube1024 with the packets: 189.7 -> 187.5 ms).  With one factor for the three channels, the pdfs' products by
+// reciprocals and these from the special function unit's flushing form it took 3 ms less, but pdfs below the
+// normal range gave black, and the error against FP64 was up to 5 % larger.  As it is, the L2 error over six
+// scenes and three seeds is 0.91 to 1.001 times the general form's.
 template <bool kDirect>
 __device__ __forceinline__ Rgb bb1d_contrib_packed(const GatherConsts& K, const DMedium& m, const SegCtx& s,
                                                    const PiecePayload& py, const PairGeo& g, float radius)
@@ -362,12 +361,9 @@ __device__ __forceinline__ Rgb bb1d_contrib_packed(const GatherConsts& K, const 
     constexpr float inv4pi = (1.f / UPBP_PI_F) * 0.25f;
     const float phase =
         fabsf(m.g) < 1e-3f ? inv4pi : (hd > 0.f ? inv4pi * (1.f - g2) / (hd * sqrtf(hd)) : 0.f);
-    // one factor for the three channels.  The root and the kernel are as in the general form: with the two
-    // functions' product rcp(hd) rsqrt(hd) and (1 - x)(1 + x) * 0.75 / (r sin), 1.8 % faster, each rounding of a
-    // constant goes the same way for every pair, and the error against FP64 grew by up to 6.6 % (SHORT query
-    // beams), 3.1 % (nested boxes) and 1.2 % (cube128); now it is within 0.4 % to either side, 1.7 % for the first
-    const float scale = phase * (1.f - g.dist * g.dist / (radius * radius)) * 3.f / (4.f * radius * g.sinT);
-    const Rgb unweighted = Rgb{py.thr.x * m.ss[0], py.thr.y * m.ss[1], py.thr.z * m.ss[2]} * att * scale;
+    const Rgb ss{m.ss[0], m.ss[1], m.ss[2]};
+    const Rgb unweighted = (Rgb{py.thr.x, py.thr.y, py.thr.z} * ss * att * phase * (1.f - g.dist * g.dist / (radius * radius))) * 3.f /
+                           (4.f * radius * g.sinT);
     if (P.techniques & UPBP_NO_MIS) return unweighted;
     const int L = kDirect ? 1 : s.L;
     const uint32_t length = (uint32_t)((int)(lvbits & kPayPathMask) + 1 + L);
@@ -383,20 +379,22 @@ __device__ __forceinline__ Rgb bb1d_contrib_packed(const GatherConsts& K, const 
     rsrB *= py.pdf.y;
     const float ratio = 1.0f / m.min_st;
     const float bsdfPdfW = phase * m.cont;
-    const float rspInvQ = fast_rcp(rspQ), rspInvB = fast_rcp(rspB);
+    const float rspInvQ = 1.0f / rspQ, rspInvB = 1.0f / rspB;
     const float distSqQ = g.t1 * g.t1, distSqB = (lvbits & kPayFinite) ? g.u * g.u : 1.0f;
     const bool no_sine = (s.ray_flags & UPBP_NO_SINE_IN_WEIGHTS) != 0;
     upbp_mis cand;
     fill_cand(cand, P, s.last_pdf_w_inv * distSqQ * rspInvQ, rspInvQ, ratio, 1.0f, UPBP_MIS_IN_MEDIUM_WITH_BEAMS);
-    // last = rsp of the LONG beams, 1 / sigma_t of the SHORT ones, over the BB1D factor and the sine
     const float sinT = no_sine ? 1.0f : g.sinT;
-    const float last = (qshort ? m.min_st : rspQ) * (bshort ? m.min_st : rspB) * fast_rcp(P.mis_factor_bb1d * sinT);
+    const float f = P.mis_factor_bb1d;
+    float last;
+    if (qshort) last = bshort ? (float)(1.0 / (double)(ratio * ratio * f * sinT)) : rspB / (ratio * f * sinT);
+    else last = bshort ? rspQ / (ratio * f * sinT) : rspQ * rspB / (f * sinT);
     const float wc = camera_weight_fast(L, cand, last, sinT, rspInvB, ratio, bsdfPdfW * rsrQ / distSqQ, *s.e, 1.0f / rsrQ,
                                         *s.cs, s.ray_flags, P.query_beam_type, P.photon_beam_type);
     float inner = distSqB * py.lv.y;
     if (!(s.ray_flags & UPBP_PREVIOUS)) inner += bsdfPdfW * py.lv.x * (py.thr.w * rsrB + py.pdf.w);
     const float wl = last * py.pdf.z * rspInvB * inner;
-    return fast_rcp(wl + wc) * unweighted;
+    return (1.0f / (wl + wc)) * unweighted;
 }
 
 // ----------------------------------------------------------------- segment loop
