@@ -234,7 +234,7 @@ __device__ __forceinline__ int pair_slow(V3 O1, V3 d1, float dmin, float dmax, V
     if (radius_at(rs, rc, t2) < dist) return 0;  // PhotonBeam.hxx:411-413
     if (!piece_takes(O1, d1, dmin, dmax, O2, d2, len, t_lo, t_hi, t1, b, e, dist, rs, rc, extra)) return 0;
     if (1.f - b * b < 1e-2f) closest_approach_f64(O1, d1, O2, d2, dist, sinT, t1, t2);
-    g = PairGeo{b, dist, sinT, t1, t2};
+    g = PairGeo{b, dist * dist, sinT, t1, t2};
     return 1;
 }
 
@@ -362,7 +362,7 @@ __device__ __forceinline__ Rgb bb1d_contrib_packed(const GatherConsts& K, const 
     const float phase =
         fabsf(m.g) < 1e-3f ? inv4pi : (hd > 0.f ? inv4pi * (1.f - g2) / (hd * sqrtf(hd)) : 0.f);
     const Rgb ss{m.ss[0], m.ss[1], m.ss[2]};
-    const Rgb unweighted = (Rgb{py.thr.x, py.thr.y, py.thr.z} * ss * att * phase * (1.f - g.dist * g.dist / (radius * radius))) * 3.f /
+    const Rgb unweighted = (Rgb{py.thr.x, py.thr.y, py.thr.z} * ss * att * phase * (1.f - g.d2 / (radius * radius))) * 3.f /
                            (4.f * radius * g.sinT);
     if (P.techniques & UPBP_NO_MIS) return unweighted;
     const int L = kDirect ? 1 : s.L;

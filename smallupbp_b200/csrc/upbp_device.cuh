@@ -296,14 +296,16 @@ __device__ __forceinline__ bool piece_takes_f64(V3 O1, V3 d1, float dmin, float 
 // The candidate decision and the closest approach of one pair, for the mixed mode's packets: 1 = this piece
 // takes the pair, 0 = it does not, -1 = undecided (the exact radius test and the reach rule decide; nearly
 // parallel pairs too, which also need the FP64 closest approach).  The predicate and its t1 and t2 are
-// test_beam_beam's operations; d1O1 = d1.O1 is the ray's, w = O2 - O1.  The distance and the sine come from
-// one approximate reciprocal square root instead of a root and a division, so the radius test is left
+// test_beam_beam's operations; d1O1 = d1.O1 is the ray's, w = O2 - O1.  For the tests the distance and the sine
+// come from one approximate reciprocal square root instead of a root and a division, so the radius test is left
 // open within errb of the radius (the bound of piece_takes_fast, twice) and in the last 0.3 % of it, where
-// the kernel 1 - d^2 / r^2 would magnify their rounding; the owner is decided as there, and the reach rule
+// the kernel 1 - d^2 / r^2 magnifies rounding.  The kernel takes the squared distance from one division, without the
+// root, and the contribution the IEEE root for the sine (with an IEEE division by it for the distance as well 188.4
+// instead of 184.4 ms at cube1024); the owner is decided as there, and the reach rule
 // holds: the closest points lie inside both segments.  scale: the largest coordinate or
 // length in play; w1 bounds |w|_1; the directions are of unit length to 2e-6.
 struct PairGeo {
-    float cosb, dist, sinT, t1, u;  // d1.d2, distance, sin(theta), the lines' parameters
+    float cosb, d2, sinT, t1, u;  // d1.d2, squared distance, sin(theta), the lines' parameters
 };
 __device__ __forceinline__ int bb1d_pair_fast(V3 O1, V3 d1, float d1O1, float dmin, float dmax, V3 O2, V3 d2, float len,
                                               float r2max, float t_lo, float t_hi, float w1, float scale, float rs,
@@ -324,8 +326,8 @@ __device__ __forceinline__ int bb1d_pair_fast(V3 O1, V3 d1, float d1O1, float dm
     if (t2 <= 0.f || t2 >= len || isnan(t2)) return 0;
     const float rsn = fast_rsqrt(s2), dist = fabsf(ad) * rsn;
     g.cosb = b;
-    g.dist = dist;
-    g.sinT = s2 * rsn;
+    g.sinT = __fsqrt_rn(s2);
+    g.d2 = ad * ad / s2;
     g.t1 = t1;
     g.u = t2;
     const float m = 6e-6f * scale * (rsn * rsn);

@@ -331,6 +331,17 @@ __device__ __forceinline__ void packet_test(const GatherConsts& K, const BeamBVH
     S.mask[first >> 5][lane] = word;
 }
 
+// A load that stays where it is written: what only the contribution needs is read there, or it would take the
+// pair's registers (cube1024 193.2 -> 187.9 ms).
+__device__ __forceinline__ float4 ld_shared(const float4* p)
+{
+    float4 v;
+    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+                 : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+                 : "r"((unsigned)__cvta_generic_to_shared(p)));
+    return v;
+}
+
 // One ray, lane = piece: evaluates the pieces that it can meet, 32 at a time.  Pairs that FP32 does not
 // decide (2 % of them) wait in the ray's list until there are 32, or until the segment ends (flush): the
 // exact predicate, the FP64 closest points and their divergence are paid for once in 32 pairs.
@@ -365,9 +376,6 @@ __device__ __forceinline__ void packet_ray(const GatherConsts& K, const LightSoA
         s.d = v3(rd.x, rd.y, rd.z);
         s.dmin = rd.w;
         s.dmax = rs.x;
-        s.rs_pdf = rs.y;
-        s.rs_rev_pdf = rs.z;
-        s.last_pdf_w_inv = rs.w;
         s.rsf = (uint32_t)S.ray_i[r] >> 8;
         s.L = 1;
         s.ray_flags = K.P.query_beam_type | K.P.techniques;
@@ -380,7 +388,6 @@ __device__ __forceinline__ void packet_ray(const GatherConsts& K, const LightSoA
     Rgb part = rgb(0.f);
     unsigned cnt = 0;
     unsigned long long h = 0;
-    const float scale = S.walk.scale, d1O1 = xdot3(s.d, s.o);
     int base = 0;
     for (;;) {
         // the slow list first when it is full (or at the end); its order in the sum is fixed as well
@@ -421,8 +428,9 @@ __device__ __forceinline__ void packet_ray(const GatherConsts& K, const LightSoA
                     take = pair_slow(s.o, s.d, s.dmin, s.dmax, o2, d2, pa.w, pb.w, pc.x, pc.y, rs, rc, K.bb1d_extra, pg);
                     hp = mix64((unsigned long long)beam);
                 } else {
-                    take = bb1d_pair_fast(s.o, s.d, d1O1, s.dmin, s.dmax, o2, d2, pa.w, pb.w, pc.x, pc.y, S.walk.reach,
-                                          fmaxf(scale, pa.w), rs, rc, pg);
+                    // d1.O1 and the scale are taken anew, for the registers (cube1024 187.9 -> 184.8 ms)
+                    take = bb1d_pair_fast(s.o, s.d, xdot3(s.d, s.o), s.dmin, s.dmax, o2, d2, pa.w, pb.w, pc.x, pc.y,
+                                          S.walk.reach, fmaxf(S.walk.scale, pa.w), rs, rc, pg);
                     if (!unit) take = -1;
                 }
             } else {
@@ -443,7 +451,11 @@ __device__ __forceinline__ void packet_ray(const GatherConsts& K, const LightSoA
                 ++cnt;
                 h += hp;
                 const float radius = radius_at(rs, rc, pg.u);
-                if (kMixed) {  // loaded here for the registers: 186 -> 175 ms at cube1024
+                const float4 rs4 = ld_shared(&S.ray_s[r]);  // dmax, mRaySamplePdf, mRaySampleRevPdf, last_pdf_w_inv
+                s.rs_pdf = rs4.y;
+                s.rs_rev_pdf = rs4.z;
+                s.last_pdf_w_inv = rs4.w;
+                if (kMixed) {  // loaded here for the registers as well
                     py.thr = __ldg(&B.pay[piece].thr);
                     py.pdf = __ldg(&B.pay[piece].pdf);
                     part = part + bb1d_contrib_packed<true>(K, m, s, py, pg, radius);
