@@ -265,8 +265,10 @@ struct PacketShared {
     float4 ray_d[32];            // direction, dmin
     float4 ray_s[32];            // dmax, mRaySamplePdf, mRaySampleRevPdf, last_pdf_w_inv
     int ray_i[32];               // medium | raySamplingFlags << 8
-    // per ray: the result, in the segment and of all segments
-    float acc_r[32], acc_g[32], acc_b[32], sum_r[32], sum_g[32], sum_b[32];
+    // per ray: the result, in the segment (the rounds' sums, in FP64: a running FP32 sum of them would round more
+    // than the 32 sums of a warp's lanes do) and of all segments
+    double acc_r[32], acc_g[32], acc_b[32];
+    float sum_r[32], sum_g[32], sum_b[32];
     unsigned cnt[32];
     unsigned long long hash[32];
     // the pieces in hand: which, their candidate hash, and per 32 of them and ray those the ray can meet
@@ -728,7 +730,7 @@ __device__ __forceinline__ void packet_segment(const GatherConsts& K, const SegQ
         S.leaves[0] = S.stack[0] = 0;
         S.next_ray = 0;
     }
-    S.acc_r[lane] = S.acc_g[lane] = S.acc_b[lane] = 0.f;
+    S.acc_r[lane] = S.acc_g[lane] = S.acc_b[lane] = 0.0;
     S.slow_n[lane] = 0;
 }
 
@@ -796,9 +798,9 @@ k_bb1d_packet(const __grid_constant__ GatherConsts K, const __grid_constant__ Li
             // (a ray whose segments have ended may hold an attenuation that is no number, which segment_loop
             // never uses)
             if (warp == 0 && (S.walk.active >> lane & 1u)) {
-                S.sum_r[lane] += S.attn_r[lane] * S.acc_r[lane];
-                S.sum_g[lane] += S.attn_g[lane] * S.acc_g[lane];
-                S.sum_b[lane] += S.attn_b[lane] * S.acc_b[lane];
+                S.sum_r[lane] += S.attn_r[lane] * (float)S.acc_r[lane];
+                S.sum_g[lane] += S.attn_g[lane] * (float)S.acc_g[lane];
+                S.sum_b[lane] += S.attn_b[lane] * (float)S.acc_b[lane];
             }
             __syncthreads();
         }
