@@ -166,7 +166,7 @@ __device__ __forceinline__ Rgb bb1d_query_warp(const GatherConsts& K, const DMed
             const int beam = __float_as_int(pc.z);
             if (kMixed) {
                 const PiecePayload py = B.pay[i];
-                const PairGeo pg{s.d.x * pb.x + s.d.y * pb.y + s.d.z * pb.z, g.x * g.x, g.y, g.z, g.w};
+                const PairGeo pg{xdot3(s.d, v3(pb.x, pb.y, pb.z)), g.x * g.x, g.y, g.z, g.w};
                 part = part + bb1d_contrib_packed<false>(K, m, s, py, pg, beam_radius_at(Bs, beam, py.lv.z, g.w));
             } else {
                 part = part + bb1d_contrib<false>(K, m, Lv, Bs, s, beam, v3(pa.x, pa.y, pa.z), v3(pb.x, pb.y, pb.z),
@@ -1001,7 +1001,7 @@ __device__ __forceinline__ Rgb bb1d_query_grid(const GatherConsts& K, const DMed
                 // (the candidate decision above stays FP32)
                 const float cb = s.d.x * d2.x + s.d.y * d2.y + s.d.z * d2.z;
                 if (1.f - cb * cb < 1e-2f) closest_approach_f64(s.o, s.d, o2, d2, dist, sinT, t1, t2);
-                c = bb1d_contrib_packed<false>(K, m, s, G.pay[b], PairGeo{cb, dist * dist, sinT, t1, t2},
+                c = bb1d_contrib_packed<false>(K, m, s, G.pay[b], PairGeo{xdot3(s.d, d2), dist * dist, sinT, t1, t2},
                                                beam_radius_at(Bs, b, rs, t2));
             } else {
                 c = bb1d_contrib<false>(K, m, Lv, Bs, s, b, o2, d2, radius, dist, sinT, t1, t2);
