@@ -140,9 +140,6 @@ struct upbp_ctx {
     int build_launches = 0, eval_launches = 0;
     float t_build = 0.f, t_pp3d = 0.f, t_pb2d = 0.f, t_bb1d = 0.f;
     cudaEvent_t ev[8] = {};
-    // the BB1D gather of the queries outside packets runs beside the packets' (created at first use)
-    cudaStream_t side_stream = nullptr;
-    cudaEvent_t fork = nullptr, join = nullptr;
 };
 
 namespace {
@@ -1173,12 +1170,6 @@ void do_evaluate(upbp_ctx* c)
         bb_order = c->bb_order.as<int32_t>();
         c->eval_launches += 4;
     }
-    if (packets) {
-        if (!c->side_stream) ck(c, cudaStreamCreateWithFlags(&c->side_stream, cudaStreamNonBlocking), "stream");
-        if (!c->fork) ck(c, cudaEventCreateWithFlags(&c->fork, cudaEventDisableTiming), "event");
-        if (!c->join) ck(c, cudaEventCreateWithFlags(&c->join, cudaEventDisableTiming), "event");
-        ck(c, cudaEventRecord(c->fork, s), "fork");
-    }
     if (nq > 0) {
         const BeamBVH B = beam_bvh(c);
         const BeamSoA S = beam_soa(c);
@@ -1197,21 +1188,16 @@ void do_evaluate(upbp_ctx* c)
             record_status(c, s);
         } else if (c->bb1d_kernel >= 1) {
             const int grid = c->num_sms * bb1d_warp_blocks_per_sm(mixed, c->bb1d_kernel);
-            if (packets) {
-                // The two gathers share no query.  The second stream lets the blocks of the per-query gather
-                // take the SMs that the last packets leave idle.
+            if (packets) {  // the two gathers share no query, and the second starts beside the first
                 launch_bb1d_packet(K, L, B, S, Q, O, order, PK, c->bbox_pc.as<float>(), piece_len, packet_grid, mixed,
                                    c->work.as<unsigned int>() + 3, s);
                 c->eval_launches += 1;
-                ck(c, cudaStreamWaitEvent(c->side_stream, c->fork, 0), "fork");
-                launch_bb1d_warp(K, L, B, S, Q, cam, cs_seg, O, grid, mixed, c->work.as<unsigned int>(),
-                                 c->status.as<int>(), bb_order, c->side_stream, c->bb1d_kernel, &PK.totals->queries);
-                ck(c, cudaEventRecord(c->join, c->side_stream), "join");
-                ck(c, cudaStreamWaitEvent(s, c->join, 0), "join");
-            } else {
-                launch_bb1d_warp(K, L, B, S, Q, cam, cs_seg, O, grid, mixed, c->work.as<unsigned int>(),
-                                 c->status.as<int>(), bb_order, s, c->bb1d_kernel, nullptr);
             }
+            ck(c,
+               launch_bb1d_warp(K, L, B, S, Q, cam, cs_seg, O, grid, mixed, c->work.as<unsigned int>(),
+                                c->status.as<int>(), bb_order, s, c->bb1d_kernel,
+                                packets ? &PK.totals->queries : nullptr),
+               "BB1D gather");
             record_status(c, s);
         } else {
             launch_gather_bb1d(K, L, B, S, Q, cam, cs_seg, O, c->block, mixed, s);
@@ -1306,9 +1292,6 @@ int upbp_ctx_destroy(upbp_ctx* c)
     if (c->status_host) cudaFreeHost(c->status_host);
     for (auto& e : c->ev)
         if (e) cudaEventDestroy(e);
-    if (c->fork) cudaEventDestroy(c->fork);
-    if (c->join) cudaEventDestroy(c->join);
-    if (c->side_stream) cudaStreamDestroy(c->side_stream);
     if (c->own_stream) cudaStreamDestroy(c->own_stream);
     delete c;
     return UPBP_OK;

@@ -329,7 +329,8 @@ __device__ __forceinline__ Rgb pb2d_query_warp(const GatherConsts& K, const DMed
 
 // BB1D, warp per query, persistent: warps draw query indices (in Morton order of the query
 // midpoints) from an atomic counter.  elsewhere: how many queries at the end of the order the packet
-// gather evaluates (NULL: none).
+// gather evaluates (NULL: none).  The launch may overlap that gather's, whose results nothing here reads; every
+// block waits for its end, so that what follows in the stream follows both.
 template <bool kMixed, int kWarps, int kMinBlocks>
 __global__ void __launch_bounds__(kWarps * 32, kMinBlocks) k_bb1d_warp(const __grid_constant__ GatherConsts K, const LightSoA Lv,
                                                           const BeamBVH B, const BeamSoA Bs, const SegQueriesDev Q,
@@ -379,6 +380,7 @@ __global__ void __launch_bounds__(kWarps * 32, kMinBlocks) k_bb1d_warp(const __g
             if (O.tested) atomicAdd(O.tested, tested);
         }
     }
+    asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
 // PB2D, warp per query, persistent (the BB1D kernel's scheme over the photon LBVH): the lanes
@@ -1276,19 +1278,28 @@ int bb1d_warp_blocks_per_sm(bool mixed, int variant)
     return mixed ? blocks_for<true>(variant) : blocks_for<false>(variant);
 }
 
-void launch_bb1d_warp(const GatherConsts& K, const LightSoA& L, const BeamBVH& B, const BeamSoA& S,
-                      const SegQueriesDev& Q, const upbp_mis* cam, const CamSum* cs, const Outputs& O, int grid,
-                      bool mixed, unsigned int* work, int* status, const int32_t* order, cudaStream_t stream,
-                      int variant, const unsigned* elsewhere)
+// Behind the packet gather (elsewhere) this one may start as soon as all blocks of that run: its blocks take what
+// the last packets leave idle.  On a second stream they did so too, but there the kernel waited for room in a
+// hardware queue that another context's stream may share, and held up that one's build: two contexts
+// in turn took 194.5 or 203.6 ms per step at cube1024, by the luck of the streams' queues, now 194.4.
+cudaError_t launch_bb1d_warp(const GatherConsts& K, const LightSoA& L, const BeamBVH& B, const BeamSoA& S,
+                             const SegQueriesDev& Q, const upbp_mis* cam, const CamSum* cs, const Outputs& O, int grid,
+                             bool mixed, unsigned int* work, int* status, const int32_t* order, cudaStream_t stream,
+                             int variant, const unsigned* elsewhere)
 {
-    if (Q.n <= 0) return;
-    if (variant == 2) {
-        if (mixed) k_bb1d_warp<true, 4, 7><<<grid, 128, 0, stream>>>(K, L, B, S, Q, cam, cs, O, work, status, order, elsewhere);
-        else k_bb1d_warp<false, 4, 7><<<grid, 128, 0, stream>>>(K, L, B, S, Q, cam, cs, O, work, status, order, elsewhere);
-    } else {
-        if (mixed) k_bb1d_warp<true, 4, 6><<<grid, 128, 0, stream>>>(K, L, B, S, Q, cam, cs, O, work, status, order, elsewhere);
-        else k_bb1d_warp<false, 4, 6><<<grid, 128, 0, stream>>>(K, L, B, S, Q, cam, cs, O, work, status, order, elsewhere);
-    }
+    if (Q.n <= 0) return cudaSuccess;
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3(128);
+    cfg.stream = stream;
+    cfg.attrs = &attr;
+    cfg.numAttrs = elsewhere ? 1 : 0;
+    auto* f = variant == 2 ? (mixed ? k_bb1d_warp<true, 4, 7> : k_bb1d_warp<false, 4, 7>)
+                           : (mixed ? k_bb1d_warp<true, 4, 6> : k_bb1d_warp<false, 4, 6>);
+    return cudaLaunchKernelEx(&cfg, f, K, L, B, S, Q, cam, cs, O, work, status, order, elsewhere);
 }
 
 namespace {

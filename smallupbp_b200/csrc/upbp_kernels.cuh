@@ -290,10 +290,11 @@ void launch_mt64_floats(unsigned long long seed, int64_t n, float* out, cudaStre
 void launch_grid_reduce(const uint32_t* cells, uint32_t n_cells, uint32_t max_beams, uint32_t reduction,
                         const uint32_t* draw_off, const float* rnd, int32_t* ptr, float* pdf, cudaStream_t s);
 
-void launch_bb1d_warp(const GatherConsts& K, const LightSoA& L, const BeamBVH& B, const BeamSoA& S,
-                      const SegQueriesDev& Q, const upbp_mis* cam, const CamSum* cs, const Outputs& O, int grid,
-                      bool mixed, unsigned int* work, int* status, const int32_t* order, cudaStream_t stream,
-                      int variant, const unsigned* elsewhere);
+// elsewhere: with packets, how many queries they hold (on the device); the launch then follows theirs directly
+cudaError_t launch_bb1d_warp(const GatherConsts& K, const LightSoA& L, const BeamBVH& B, const BeamSoA& S,
+                             const SegQueriesDev& Q, const upbp_mis* cam, const CamSum* cs, const Outputs& O, int grid,
+                             bool mixed, unsigned int* work, int* status, const int32_t* order, cudaStream_t stream,
+                             int variant, const unsigned* elsewhere);
 void launch_gather_bp2d(const GatherConsts& K, const BeamBVH& B, const BeamSoA& S, const PointQueriesDev& Q,
                         const Outputs& O, int block, cudaStream_t stream);
 int bp2d_warp_blocks_per_sm();

@@ -746,6 +746,7 @@ k_bb1d_packet(const __grid_constant__ GatherConsts K, const __grid_constant__ Li
 {
     extern __shared__ __align__(16) unsigned char smem[];
     PacketShared& S = *reinterpret_cast<PacketShared*>(smem);
+    asm volatile("griddepcontrol.launch_dependents;");  // the gather per query may start beside this one
     stage_media(K, S.media);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     for (;;) {
