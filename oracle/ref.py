@@ -29,6 +29,10 @@ class RefOutputs(C.Structure):
 _lib = None
 
 
+class NotBuilt(FileNotFoundError):
+    """The reference library is not there (tests that call it are skipped)."""
+
+
 def available() -> bool:
     return os.path.exists(LIB_PATH)
 
@@ -37,7 +41,7 @@ def lib():
     global _lib
     if _lib is None:
         if not available():
-            raise FileNotFoundError(LIB_PATH + " is not built (python oracle/build_ref.py)")
+            raise NotBuilt(LIB_PATH + " is not built (python oracle/build_ref.py)")
         _lib = C.CDLL(LIB_PATH)
         _lib.ref_run.restype = C.c_int
         _lib.ref_run.argtypes = [C.POINTER(abi.Params), C.POINTER(abi.Medium), C.c_int32,
