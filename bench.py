@@ -224,8 +224,8 @@ def kernel_source_hash() -> str:
     import hashlib
     h = hashlib.sha256()
     csrc = os.path.join(ROOT, "smallupbp_b200", "csrc")
-    for f in ("upbp_gather.cu", "upbp_device.cuh", "upbp_traverse.cuh", "upbp_kernels.cuh", "upbp_build.cu",
-              "upbp_capi.cu"):
+    for f in ("upbp_gather.cu", "upbp_packet.cu", "upbp_contrib.cuh", "upbp_device.cuh", "upbp_traverse.cuh",
+              "upbp_kernels.cuh", "upbp_build.cu", "upbp_capi.cu"):
         with open(os.path.join(csrc, f), "rb") as fh:
             h.update(fh.read())
     return h.hexdigest()[:16]

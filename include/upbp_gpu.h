@@ -385,7 +385,10 @@ int upbp_read_bp2d_results(upbp_ctx* ctx, float* rgb, uint32_t* count, uint64_t*
 int upbp_device_bytes(const upbp_ctx* ctx, uint64_t* bytes);
 
 /* Candidates tested by the last evaluate, summed over all queries: [0] PB2D photons, [1] BB1D beam
- * pieces, [2] PP3D photons (diagnostics of culling quality; accepted counts are in the query stats). */
+ * pieces, [2] PP3D photons (diagnostics of culling quality; accepted counts are in the query stats).
+ * [1] counts (query, piece) pairs whose first check ran: every piece of the leaves that a query's own
+ * walk visits and, for the camera rays that are evaluated in packets, every piece that its packet's
+ * walk keeps, once per ray with a segment in hand. */
 int upbp_read_tested_counts(upbp_ctx* ctx, uint64_t* tested);
 int upbp_clear_image(upbp_ctx* ctx); /* zeroes the framebuffer and the per-query results */
 int upbp_read_image(upbp_ctx* ctx, float* rgb); /* [H*W][3] accumulated */

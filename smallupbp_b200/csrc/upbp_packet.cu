@@ -11,15 +11,16 @@
 // sums in registers.  (A lane per ray instead had 31 of 100 lanes busy, as the rays' work differs, and
 // dealing the pairs evenly paid as much for moving between rays.)
 //
-// What bounds it: instructions.  At cube512 6.7 G instructions for 226 M accepted pairs, half of them in
-// the evaluation, issued in 0.6 of the cycles; 24 warps per SM at 80 registers, little from DRAM.  BB1D
-// with the per-query gather beside it (mixed mode), against that gather alone: cube1024 262.8 -> 175.5 ms,
-// boxes3 417.8 -> 288.5 ms, cube512 20.7 -> 15.6 ms, the same with KNN radii 12.4 -> 9.5 ms; plain mode
-// at cube512 33.8 -> 27.4 ms.
+// What bounds it: instructions, issued in 0.65 of the cycles (ncu, cube512: 7.2 G for 226 M accepted pairs); 24
+// warps per SM at 80 registers, and every register that its inner loops spill costs: the L1 that three
+// blocks leave is small.  BB1D with the per-query gather beside it (mixed mode), against that gather alone: cube1024
+// 269.2 -> 185.4 ms, boxes3 426.6 -> 305.3 ms, cube512 21.2 -> 16.3 ms, the same with KNN radii 12.3 -> 9.8 ms;
+// plain mode at cube512 33.5 -> 27.9 ms, at cube1024 542.9 -> 420.4 ms.
 //
 // The candidate set is the one of the per-query kernels: every accepted pair passes the reference's FP32
 // predicate (PhotonBeam.hxx:238-296), the radius test and the reach rule (upbp_device.cuh); the checks
-// before them are conservative.
+// before them are conservative.  The values are theirs too, but for the rounding of the squared distance
+// (bb1d_pair_fast) and of the sums.
 #include <algorithm>
 #include <cfloat>
 #include <cstdint>
@@ -205,7 +206,7 @@ __global__ void __launch_bounds__(256) k_packet_setup(const SegQueriesDev Q, con
 // all work (the heaviest packet has 15 times the mean's work, and in a small image a packet's block
 // would run long after the others are done).  Each item is a packet of its own, with a narrower frustum,
 // but walks the tree again: at cube512 a share of 0.05 / 0.25 / 0.6 / 1 of what a resident block gets
-// on average took 18.4 / 15.7 / 14.9 / 15.0 ms.  The items are sorted by weight; slots without one have 0 (the
+// on average took 18.4 / 15.7 / 14.9 / 15.0 ms (an earlier version).  The items are sorted by weight; slots without one have 0 (the
 // caller's).  A packet of P parts has more than share P / 2 of the weight, so that there are at most
 // 2 / share items more than packets.
 __global__ void __launch_bounds__(256) k_packet_items(const uint32_t* __restrict__ weight, const int2* __restrict__ range,
@@ -812,7 +813,8 @@ k_bb1d_packet(const __grid_constant__ GatherConsts K, const __grid_constant__ Li
     }
 }
 
-constexpr int kPBlocks = 3;  // measured at cube1024: 2 blocks 228 ms, 3 190, 4 (512-piece rounds) 193
+// BB1D at cube1024: 2 blocks 215 ms, 3 185; 4 (with rounds of 512 pieces, an earlier version) 193 against 190
+constexpr int kPBlocks = 3;
 
 template <bool kMixed>
 int blocks_per_sm()

@@ -322,7 +322,8 @@ class EstimatorStage:
         return np.array(list(out), np.float64)
 
     def tested_counts(self):
-        """Candidates tested by the last evaluate: {"pb2d": photons, "bb1d": beam pieces, "pp3d": photons}."""
+        """Candidates tested by the last evaluate: {"pb2d": photons, "bb1d": beam pieces, "pp3d": photons}; rays
+        in packets test the pieces that their packet's walk keeps, the other queries those of the leaves they visit."""
         out = np.zeros(3, np.uint64)
         self._ck(self._l.upbp_read_tested_counts(self._ctx, abi.ptr(out)))
         return {"pb2d": int(out[0]), "bb1d": int(out[1]), "pp3d": int(out[2])}

@@ -1,4 +1,4 @@
-"""The packets' gather and the gather per query beside it (an iteration of 100,000 segment queries and more): on a
+"""The packets' gather and the gather per query beside it (an iteration of 80,000 camera queries and more): on a
 caller's stream, in a captured graph, and in two contexts at once.  The values per query do not depend on
 which of the two gathers runs when, so they are equal bit for bit."""
 import numpy as np
