@@ -945,9 +945,8 @@ __device__ __forceinline__ bool grid_maybe(const float (*ray)[8], float4 line, f
 //
 // Bound by instruction issue and the loads' latency: at cube512 over a 64^3 grid a query checks 15,000 entries
 // and takes 1,260.  With the cells queued in shared memory, two 16-byte loads per entry, the predicate's own
-// checks and batches that ended with the queue 37.0 ms, now 29.6 ms (128^3: 37.3 -> 33.0, cube128 over 64^3:
-// 1.06 -> 0.76; mixed mode).  Cells' last entries as partly filled batches: 31.8 instead of 29.0 ms (an earlier
-// version of the contribution).
+// checks and batches that ended with the queue 35.7 ms, now 29.0 ms (128^3: 36.3 -> 32.4, cube128 over 64^3:
+// 1.00 -> 0.76).  Cells' last entries as partly filled batches: 31.8 ms.
 template <bool kMixed>
 __device__ __forceinline__ Rgb bb1d_query_grid(const GatherConsts& K, const DMedium* media, const LightSoA& Lv,
                                                const BeamGrid& G, const GridHeader& hdr, const BeamSoA& Bs,
@@ -1101,11 +1100,11 @@ __device__ __forceinline__ Rgb bb1d_query_grid(const GatherConsts& K, const DMed
     return res;
 }
 
-// Persistent, one warp per query from the atomic work queue.  Blocks of 4 warps per SM, by what their spills cost: at
-// cube512 over a 64^3 and a 128^3 grid and at cube128 over 64^3, mixed mode 4 blocks 29.6, 33.0 and 0.76 ms, 5 29.8,
-// 33.8 and 0.81, 6 31.0, 35.2 and 0.84; plain mode 42.1, 46.9 and 0.94, 40.7, 46.6 and 0.97, 43.2, 49.4 and 1.07.
+// Persistent, one warp per query from the atomic work queue.  5 blocks of 4 warps per SM: 6 and 7, with more
+// spills, take 29.1 and 29.6 ms instead of 29.0 at cube512 over a 64^3 grid, 0.78 and 0.81 instead of 0.76 at
+// cube128.
 template <bool kMixed>
-__global__ void __launch_bounds__(128, kMixed ? 4 : 5) k_bb1d_grid(const __grid_constant__ GatherConsts K, const LightSoA Lv,
+__global__ void __launch_bounds__(128, 5) k_bb1d_grid(const __grid_constant__ GatherConsts K, const LightSoA Lv,
                                                   const BeamGrid G, const BeamSoA Bs, const SegQueriesDev Q,
                                                   const upbp_mis* __restrict__ cam, const CamSum* __restrict__ cs,
                                                   const Outputs O, unsigned int* __restrict__ work,
