@@ -945,8 +945,9 @@ __device__ __forceinline__ bool grid_maybe(const float (*ray)[8], float4 line, f
 //
 // Bound by instruction issue and the loads' latency: at cube512 over a 64^3 grid a query checks 15,000 entries
 // and takes 1,260.  With the cells queued in shared memory, two 16-byte loads per entry, the predicate's own
-// checks and batches that ended with the queue 35.7 ms, now 29.0 ms (128^3: 36.3 -> 32.4, cube128 over 64^3:
-// 1.00 -> 0.76).  Cells' last entries as partly filled batches: 31.8 ms.
+// checks and batches that ended with the queue 37.0 ms, now 29.8 ms (128^3: 37.3 -> 33.8, cube128 over 64^3:
+// 1.06 -> 0.81, cube1024 over 64^3: 511 -> 399; mixed mode).  Cells' last entries as partly filled batches: 31.8
+// instead of 29.0 ms (an earlier version of the contribution).
 template <bool kMixed>
 __device__ __forceinline__ Rgb bb1d_query_grid(const GatherConsts& K, const DMedium* media, const LightSoA& Lv,
                                                const BeamGrid& G, const GridHeader& hdr, const BeamSoA& Bs,
@@ -1100,9 +1101,10 @@ __device__ __forceinline__ Rgb bb1d_query_grid(const GatherConsts& K, const DMed
     return res;
 }
 
-// Persistent, one warp per query from the atomic work queue.  5 blocks of 4 warps per SM: 6 and 7, with more
-// spills, take 29.1 and 29.6 ms instead of 29.0 at cube512 over a 64^3 grid, 0.78 and 0.81 instead of 0.76 at
-// cube128.
+// Persistent, one warp per query from the atomic work queue.  5 blocks of 4 warps per SM, between the spills of more
+// and the empty SMs of fewer: over 64^3 cells 4 / 5 / 6 blocks take 420 / 399 / 412 ms at cube1024, 726 / 681 / 698 at
+// boxes3, 29.6 / 29.8 / 31.0 at cube512 and 0.76 / 0.81 / 0.84 at cube128 (mixed mode; plain mode at cube512
+// 42.1 / 40.7 / 43.2).
 template <bool kMixed>
 __global__ void __launch_bounds__(128, 5) k_bb1d_grid(const __grid_constant__ GatherConsts K, const LightSoA Lv,
                                                   const BeamGrid G, const BeamSoA Bs, const SegQueriesDev Q,

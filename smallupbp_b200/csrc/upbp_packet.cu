@@ -11,7 +11,7 @@
 // sums in registers.  (A lane per ray instead had 31 of 100 lanes busy, as the rays' work differs, and
 // dealing the pairs evenly paid as much for moving between rays.)
 //
-// What bounds it: instructions, issued in 0.65 of the cycles (ncu, cube512: 7.2 G for 226 M accepted pairs); 24
+// What bounds it: instructions, issued in 0.67 of the cycles (ncu, cube512: 7.3 G for 226 M accepted pairs); 24
 // warps per SM at 80 registers, and every register that its inner loops spill costs: the L1 that three
 // blocks leave is small.  BB1D with the per-query gather beside it (mixed mode), against that gather alone: cube1024
 // 269.2 -> 185.4 ms, boxes3 426.6 -> 305.3 ms, cube512 21.2 -> 16.3 ms, the same with KNN radii 12.3 -> 9.8 ms;
