@@ -206,9 +206,9 @@ __global__ void __launch_bounds__(256) k_packet_setup(const SegQueriesDev Q, con
 // all work (the heaviest packet has 15 times the mean's work, and in a small image a packet's block
 // would run long after the others are done).  Each item is a packet of its own, with a narrower frustum,
 // but walks the tree again: at cube512 a share of 0.05 / 0.25 / 0.6 / 1 of what a resident block gets
-// on average took 18.4 / 15.7 / 14.9 / 15.0 ms (an earlier version).  The items are sorted by weight; slots without one have 0 (the
-// caller's).  A packet of P parts has more than share P / 2 of the weight, so that there are at most
-// 2 / share items more than packets.
+// on average took 18.4 / 15.7 / 14.9 / 15.0 ms (an earlier version).  The items are sorted by weight; slots
+// without one have 0 (the caller's).  A packet of P parts has more than share P / 2 of the weight, so that there
+// are at most 2 / share items more than packets.
 __global__ void __launch_bounds__(256) k_packet_items(const uint32_t* __restrict__ weight, const int2* __restrict__ range,
                                                       float share, unsigned slots, PacketTotals* totals, uint32_t* key,
                                                       unsigned long long* item)
